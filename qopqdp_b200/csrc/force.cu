@@ -16,7 +16,7 @@
 // atomics are needed and results are deterministic.  Everything runs in
 // FP64; the result is rounded once into the force handle's precision.
 #include "fields.cuh"
-#include "mat3.cuh"
+#include "staple.cuh"
 #include <vector>
 
 namespace qopb {
@@ -42,85 +42,117 @@ __device__ __forceinline__ void accf(double2 *f, const Geom &g, int p, int i, co
   }
 }
 
-// out = staple(in; mu, nu) = U_nu(x) in(x+nu) U_nu(x+mu)^+ + U_nu(y)^+ in(y) U_nu(y+mu), y = x-nu
-__global__ void k_fstaple(double2 *out, const double2 *in, const double2 *Unu, int mu, int nu, Geom g) {
-  const i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  int p, i, x[4], pn, in_, pm, im, py, iy, pym, iym, yy[4];
-  site_of(g, s, p, i, x);
-  nbr_pi(g, x, nu, 1, pn, in_);
-  nbr_pi(g, x, mu, 1, pm, im);
-  shifted(g, x, nu, -1, yy);
-  par_idx(g, yy, py, iy);
-  nbr_pi(g, yy, mu, 1, pym, iym);
-  M3 up = mul(ldf(Unu, g, p, i), mul_na(ldf(in, g, pn, in_), ldf(Unu, g, pm, im)));
-  M3 lo = mul(mul_an(ldf(Unu, g, py, iy), ldf(in, g, py, iy)), ldf(Unu, g, pym, iym));
+// adjoint of U_n for out += sum_k w_k staple(in_k; mu, n), with G_k the
+// adjoint of out: row r of the sum over the pairs (G, in) of
+//   G(z) U(z+mu) in(z+n)^+ + G(z-mu)^+ U(z-mu) in(z-mu+n)
+//   + in(z-mu)^+ U(z-mu) G(z-mu+n) + in(z) U(z+mu) G(z+n)^+,   U = U_n;
+// each of the two U matrices is loaded once for all pairs
+constexpr int ADJ_PAIRS = 4;
+struct AdjPairs {
+  const double2 *G[ADJ_PAIRS], *in[ADJ_PAIRS];
+  double w[ADJ_PAIRS];
+};
+__device__ __forceinline__ void adj_link_row(const Geom &g, const StSite &s, const AdjPairs &pr, int np,
+                                             const double2 *Un, int mu, int n, int r, double2 (&acc)[3]) {
+  const i64 Vh = g.Vh;
+  const int fm = st_step(g, s, mu, 1), bm = st_step(g, s, mu, -1), fn = st_step(g, s, n, 1);
+  const int p = s.p, q = 1 - p;
+  double2 u[9], x[3], t[3];
+  st_load(st_at(Un, Vh, q, s.lex + fm), Vh, u);
+#pragma unroll 1
+  for (int k = 0; k < np; k++) {
+    const double2 *const a[2] = {pr.G[k], pr.in[k]};
+    const double w = pr.w[k];
 #pragma unroll
-  for (int e = 0; e < 9; e++) up.e[e] = make_double2(up.e[e].x + lo.e[e].x, up.e[e].y + lo.e[e].y);
-  st3(out + (i64)p * 9 * g.Vh + i, g.Vh, up);
+    for (int h = 0; h < 2; h++) {   // row of a[h](z) U a[1-h](z+n)^+
+      st_row(st_at(a[h], Vh, p, s.lex), Vh, r, x);
+#pragma unroll
+      for (int c = 0; c < 3; c++) x[c] = make_double2(w * x[c].x, w * x[c].y);
+      st_mul_held(x, u, t);
+      st_mul_dag_add(t, st_at(a[1 - h], Vh, q, s.lex + fn), Vh, acc);
+    }
+  }
+  st_load(st_at(Un, Vh, q, s.lex + bm), Vh, u);
+#pragma unroll 1
+  for (int k = 0; k < np; k++) {
+    const double2 *const a[2] = {pr.G[k], pr.in[k]};
+    const double w = pr.w[k];
+#pragma unroll
+    for (int h = 0; h < 2; h++) {   // row of a[h](z-mu)^+ U a[1-h](z-mu+n)
+      st_row_dag(st_at(a[h], Vh, q, s.lex + bm), Vh, r, x);
+#pragma unroll
+      for (int c = 0; c < 3; c++) x[c] = make_double2(w * x[c].x, w * x[c].y);
+      st_mul_held(x, u, t);
+      st_mul_add(t, st_at(a[1 - h], Vh, p, s.lex + bm + fn), Vh, acc);
+    }
+  }
 }
 
-// adjoint of `in` for out += c staple(in; mu, nu):
-// Gin(z) += c [U_nu(z-nu)^+ G(z-nu) U_nu(z-nu+mu) + U_nu(z) G(z+nu) U_nu(z+mu)^+]
-__global__ void k_adj_in(double2 *Gin, const double2 *G, const double2 *Unu, int mu, int nu, double c, Geom g) {
-  const i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  int p, i, z[4], a, ai, b, bi, pn, in_, pm, im, y[4];
-  site_of(g, s, p, i, z);
-  shifted(g, z, nu, -1, y);
-  par_idx(g, y, a, ai);                 // z - nu
-  nbr_pi(g, y, mu, 1, b, bi);           // z - nu + mu
-  nbr_pi(g, z, nu, 1, pn, in_);         // z + nu
-  nbr_pi(g, z, mu, 1, pm, im);          // z + mu
-  M3 r = mul(mul_an(ldf(Unu, g, a, ai), ldf(G, g, a, ai)), ldf(Unu, g, b, bi));
-  accf(Gin, g, p, i, r, c);
-  r = mul_na(mul(ldf(Unu, g, p, i), ldf(G, g, pn, in_)), ldf(Unu, g, pm, im));
-  accf(Gin, g, p, i, r, c);
+// The derivative for one direction mu from its chains (staple.cuh): groups
+// 0-2 add the adjoint of U_n, n != mu, to D_n; group 3 adds the adjoint of
+// the starting link, c1 M + w sum_n staple(Y_n; n), to D_mu
+struct SweepArgs {
+  AdjPairs pr[3];
+  int np;
+  const double2 *M, *Y[3];
+  double2 *D[4];
+  double c1, w;
+};
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_sweep(const __grid_constant__ SweepArgs a, const __grid_constant__ StU U, int mu, Geom g) {
+  int grp, p, i;
+  if (!st_block(g, 4, grp, p, i)) return;
+  const StSite s = st_site(g, i, p);
+  const int r = threadIdx.y;
+  const i64 Vh = g.Vh;
+  double2 acc[1][3] = {};
+  int dir = mu;
+  if (grp < 3) {
+    dir = st_dir(mu, grp);
+    adj_link_row(g, s, a.pr[grp], a.np, U.d[dir], mu, dir, r, acc[0]);
+  } else {
+    st_fat_row(g, s, a.M, a.Y, U, a.c1, a.w, mu, r, acc);
+  }
+  double2 *o = st_at(a.D[dir], Vh, p, s.lex);
+#pragma unroll
+  for (int c = 0; c < 3; c++) {
+    const double2 v = o[(3 * r + c) * Vh];
+    o[(3 * r + c) * Vh] = make_double2(v.x + acc[0][c].x, v.y + acc[0][c].y);
+  }
 }
 
-// adjoint of U_nu for out += c staple(in; mu, nu):
-// GU(z) += c [G(z) U(z+mu) in(z+nu)^+ + G(z-mu)^+ U(z-mu) in(z-mu+nu)
-//             + in(z-mu)^+ U(z-mu) G(z-mu+nu) + in(z) U(z+mu) G(z+nu)^+],  U = U_nu
-__global__ void k_adj_link(double2 *GU, const double2 *G, const double2 *in, const double2 *Unu, int mu, int nu,
-                           double c, Geom g) {
-  const i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  int p, i, z[4], pm, im, pn, in_, qm, iqm, qmn, iqmn, y[4];
-  site_of(g, s, p, i, z);
-  nbr_pi(g, z, mu, 1, pm, im);          // z + mu
-  nbr_pi(g, z, nu, 1, pn, in_);         // z + nu
-  shifted(g, z, mu, -1, y);
-  par_idx(g, y, qm, iqm);               // z - mu
-  nbr_pi(g, y, nu, 1, qmn, iqmn);       // z - mu + nu
-  const M3 Upm = ldf(Unu, g, pm, im), Uqm = ldf(Unu, g, qm, iqm);
-  M3 r = mul_na(mul(ldf(G, g, p, i), Upm), ldf(in, g, pn, in_));
-  accf(GU, g, p, i, r, c);
-  r = mul(mul_an(ldf(G, g, qm, iqm), Uqm), ldf(in, g, qmn, iqmn));
-  accf(GU, g, p, i, r, c);
-  r = mul(mul_an(ldf(in, g, qm, iqm), Uqm), ldf(G, g, qmn, iqmn));
-  accf(GU, g, p, i, r, c);
-  r = mul_na(mul(ldf(in, g, p, i), Upm), ldf(G, g, pn, in_));
-  accf(GU, g, p, i, r, c);
-}
-
-// adjoint of long(x) = c U(x) U(x+mu) U(x+2mu):
+// adjoint of long(x) = c U(x) U(x+mu) U(x+2mu), the directions as groups:
 // D(z) += c [N(z) (U(z+mu) U(z+2mu))^+ + U(z-mu)^+ N(z-mu) U(z+mu)^+ + (U(z-2mu) U(z-mu))^+ N(z-2mu)]
-__global__ void k_adj_naik(double2 *D, const double2 *N, const double2 *U, int mu, double c, Geom g) {
-  const i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  int p, i, z[4], p1, i1, p2, i2, m1, j1, m2, j2;
-  site_of(g, s, p, i, z);
-  nbr_pi(g, z, mu, 1, p1, i1);
-  nbr_pi(g, z, mu, 2, p2, i2);
-  nbr_pi(g, z, mu, -1, m1, j1);
-  nbr_pi(g, z, mu, -2, m2, j2);
-  const M3 Up1 = ldf(U, g, p1, i1), Um1 = ldf(U, g, m1, j1);
-  M3 r = mul_na(ldf(N, g, p, i), mul(Up1, ldf(U, g, p2, i2)));
-  accf(D, g, p, i, r, c);
-  r = mul_na(mul_an(Um1, ldf(N, g, m1, j1)), Up1);
-  accf(D, g, p, i, r, c);
-  r = mul_an(mul(ldf(U, g, m2, j2), Um1), ldf(N, g, m2, j2));
-  accf(D, g, p, i, r, c);
+struct NaikAdjArgs {
+  double2 *D[4];
+  const double2 *N[4];
+};
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_adj_naik(const __grid_constant__ NaikAdjArgs a, const __grid_constant__ StU Us, double c, Geom g) {
+  int mu, p, i;
+  if (!st_block(g, 4, mu, p, i)) return;
+  const StSite s = st_site(g, i, p);
+  const int r = threadIdx.y, q = 1 - p;
+  const i64 Vh = g.Vh;
+  const double2 *U = Us.d[mu], *N = a.N[mu];
+  const int f1 = st_step(g, s, mu, 1), f2 = st_step(g, s, mu, 2), b1 = st_step(g, s, mu, -1),
+            b2 = st_step(g, s, mu, -2);
+  double2 x[3], t[3], o[3] = {};
+  st_row(st_at(N, Vh, p, s.lex), Vh, r, x);
+#pragma unroll
+  for (int j = 0; j < 3; j++) t[j] = make_double2(0, 0);
+  st_mul_dag_add(x, st_at(U, Vh, p, s.lex + f2), Vh, t);
+  st_row_dag(st_at(U, Vh, q, s.lex + b1), Vh, r, x);
+  st_mul_add(x, st_at(N, Vh, q, s.lex + b1), Vh, t);   // the first two terms share the last factor
+  st_mul_dag_add(t, st_at(U, Vh, q, s.lex + f1), Vh, o);
+#pragma unroll
+  for (int j = 0; j < 3; j++) t[j] = make_double2(0, 0);
+  st_mul_dag_add(x, st_at(U, Vh, p, s.lex + b2), Vh, t);
+  st_mul_add(t, st_at(N, Vh, p, s.lex + b2), Vh, o);
+  double2 *d = st_at(a.D[mu], Vh, p, s.lex);
+#pragma unroll
+  for (int j = 0; j < 3; j++) {
+    const double2 v = d[(3 * r + j) * Vh];
+    d[(3 * r + j) * Vh] = make_double2(v.x + c * o[j].x, v.y + c * o[j].y);
+  }
 }
 
 // The reference's derivative field carries, with a Lepage term, one more
@@ -335,18 +367,33 @@ __global__ void k_reunit_adj(double2 *GV, const double2 *V, const double2 *GW, i
   st3(GV + off, Vh, r);
 }
 
-// Work fields of the reverse sweep ([2][9][Vh] each)
-struct SweepWork {
-  double2 *S3, *S5, *G3, *G5;
-};
-
 // D += derivative of Re sum tr[midF^+ fat + midN^+ long] with (fat, long) =
 // make_imp_links(c, U): the reverse sweep over its staple sums and the Naik
-// products; midN may be null.  lepage_rep adds the reference's Lepage term
+// products; midN may be null.  The adjoint of a staple with respect to its
+// input is the same staple, so for every direction mu the chains of staple.cuh
+// run on U_mu (S_n, I_n = X_n with c3 = 0) and on M = midF_mu (A_n, X_n), and
+//   D_mu += c1 M + sum_n staple(X_n; n),
+//   D_n  += AL(M, I_n) + AL(X_n, U_mu) + c7 [AL(A_s, S_r) + AL(A_r, S_s)],
+// AL(G, in) the link adjoint (adj_link_row), {n, r, s} the directions != mu:
+// 12 link adjoints, 6 + 6 + 6 + 3 staples in three launches per direction.
+// Three launches and about 52 field passes per direction where walking every
+// path took 64 launches and about 300; 24^3 x 48, HISQ, 8 sources: the call
+// takes 27.0 ms against 62.1 (8^4 asqtad, 2 sources: 0.17 against 1.68).
+// The sweep kernel runs the FP64 pipe at 43 % and L1 at 51 % of their rates;
+// the latency of L2 reads at 15 warps per SM is the rest.  lepage_rep adds the reference's Lepage term
 // of the form U H (k_lep_h), for a derivative that feeds something other
-// than the force projection.  Returns the number of kernels launched.
+// than the force projection.  work: SWEEP_FIELDS fields [2][9][Vh].
+// Returns sweep_terms.
+constexpr int SWEEP_FIELDS = 12;
+// staple applications and field sums of the sweep walked path by path: the
+// unit of the flops that the force calls report
+int sweep_terms(const double c[6], bool naik, bool lepage_rep) {
+  const bool have5 = c[2] != 0 || c[3] != 0, have3 = c[1] != 0 || have5 || c[4] != 0;
+  const int per_nu = 4 + (c[4] != 0 ? 2 : 0) + (have5 ? 2 * (4 + (c[3] != 0 ? 2 : 0)) : 0);
+  return 4 * (1 + (have3 ? 3 * per_nu : 0)) + (naik && c[5] != 0 ? 4 : 0) + (lepage_rep && c[4] != 0 ? 8 : 0);
+}
 int smear_adjoint(const double2 *U, const double c[6], const double2 *mid, const double2 *midN, double2 *D,
-                  const SweepWork &w, bool lepage_rep = false) {
+                  double2 *work, bool lepage_rep = false) {
   Context &cx = ctx();
   const Geom &g = cx.g;
   const i64 F1 = 18 * g.Vh;
@@ -355,52 +402,60 @@ int smear_adjoint(const double2 *U, const double c[6], const double2 *mid, const
   const bool have5 = c5 != 0 || c7 != 0 || cL != 0, have3 = c3 != 0 || have5;
   auto Uf = [&](int d) { return U + d * F1; };
   auto Df = [&](int d) { return D + d * F1; };
+  const StU Us{{Uf(0), Uf(1), Uf(2), Uf(3)}};
   int nk = 0;
   for (int mu = 0; mu < 4; mu++) {
     const double2 *M = mid + mu * F1;
-    k_field_axpby<<<gridF, 256, 0, cx.s>>>(Df(mu), 1.0, M, c1, F1);
-    nk++;
-    if (!have3) continue;
-    for (int nu = 0; nu < 4; nu++) {
-      if (nu == mu) continue;
-      k_fstaple<<<grid2, 128, 0, cx.s>>>(w.S3, Uf(mu), Uf(nu), mu, nu, g);
-      k_field_axpby<<<gridF, 256, 0, cx.s>>>(w.G3, 0.0, M, c3, F1);
-      nk += 2;
-      if (cL != 0) {
-        k_adj_in<<<grid2, 128, 0, cx.s>>>(w.G3, M, Uf(nu), mu, nu, cL, g);
-        k_adj_link<<<grid2, 128, 0, cx.s>>>(Df(nu), M, w.S3, Uf(nu), mu, nu, cL, g);
-        nk += 2;
-      }
-      if (c5 != 0 || c7 != 0) {
-        for (int rho = 0; rho < 4; rho++) {
-          if (rho == mu || rho == nu) continue;
-          k_fstaple<<<grid2, 128, 0, cx.s>>>(w.S5, w.S3, Uf(rho), mu, rho, g);
-          k_field_axpby<<<gridF, 256, 0, cx.s>>>(w.G5, 0.0, M, c5, F1);
-          nk += 2;
-          if (c7 != 0)
-            for (int sig = 0; sig < 4; sig++) {
-              if (sig == mu || sig == nu || sig == rho) continue;
-              k_adj_in<<<grid2, 128, 0, cx.s>>>(w.G5, M, Uf(sig), mu, sig, c7, g);
-              k_adj_link<<<grid2, 128, 0, cx.s>>>(Df(sig), M, w.S5, Uf(sig), mu, sig, c7, g);
-              nk += 2;
-            }
-          k_adj_in<<<grid2, 128, 0, cx.s>>>(w.G3, w.G5, Uf(rho), mu, rho, 1.0, g);
-          k_adj_link<<<grid2, 128, 0, cx.s>>>(Df(rho), w.G5, w.S3, Uf(rho), mu, rho, 1.0, g);
-          nk += 2;
-        }
-      }
-      k_adj_in<<<grid2, 128, 0, cx.s>>>(Df(mu), w.G3, Uf(nu), mu, nu, 1.0, g);
-      k_adj_link<<<grid2, 128, 0, cx.s>>>(Df(nu), w.G3, Uf(mu), Uf(nu), mu, nu, 1.0, g);
-      nk += 2;
-    }
-  }
-  if (midN && c[5] != 0)
-    for (int mu = 0; mu < 4; mu++) {
-      k_adj_naik<<<grid2, 128, 0, cx.s>>>(Df(mu), midN + mu * F1, Uf(mu), mu, c[5], g);
+    if (!have3) {
+      k_field_axpby<<<gridF, 256, 0, cx.s>>>(Df(mu), 1.0, M, c1, F1);
       nk++;
+      continue;
     }
+    SweepArgs a{};
+    for (int d = 0; d < 4; d++) a.D[d] = Df(d);
+    a.M = M;
+    a.c1 = c1;
+    if (have5) {
+      StChain<2> ch;
+      ch.in[0] = Uf(mu);
+      ch.in[1] = M;
+      ch.c3[0] = 0;
+      ch.c3[1] = c3;
+      for (int f = 0; f < 2; f++)
+        for (int j = 0; j < 3; j++) {
+          ch.S[f][j] = work + (6 * f + j) * F1;
+          ch.X[f][j] = work + (6 * f + 3 + j) * F1;
+        }
+      k_chain_s<2><<<st_grid(g, 3), st_threads(), 0, cx.s>>>(ch, Us, mu, g);
+      k_chain_x<2><<<st_grid(g, 3), st_threads(), 0, cx.s>>>(ch, Us, StCoef{cL, c5, c7}, mu, g);
+      nk += 2;
+      a.np = c7 != 0 ? 4 : 2;
+      a.w = 1.0;
+      for (int j = 0; j < 3; j++) {
+        const int j1 = j == 0 ? 1 : 0, j2 = j == 2 ? 1 : 2;
+        a.pr[j] = AdjPairs{{M, ch.X[1][j], ch.S[1][j2], ch.S[1][j1]},
+                           {ch.X[0][j], Uf(mu), ch.S[0][j1], ch.S[0][j2]},
+                           {1.0, 1.0, c7, c7}};
+        a.Y[j] = ch.X[1][j];
+      }
+    } else {   // three-link staples only: X_n = c3 M
+      a.np = 1;
+      a.w = c3;
+      for (int j = 0; j < 3; j++) {
+        a.pr[j] = AdjPairs{{M}, {Uf(mu)}, {c3}};
+        a.Y[j] = M;
+      }
+    }
+    k_sweep<<<st_grid(g, 4), st_threads(), 0, cx.s>>>(a, Us, mu, g);
+    nk++;
+  }
+  if (midN && c[5] != 0) {
+    k_adj_naik<<<st_grid(g, 4), st_threads(), 0, cx.s>>>(
+        NaikAdjArgs{{Df(0), Df(1), Df(2), Df(3)}, {midN, midN + F1, midN + 2 * F1, midN + 3 * F1}}, Us, c[5], g);
+    nk++;
+  }
   if (lepage_rep && cL != 0) {
-    double2 *H[4] = {w.S3, w.S5, w.G3, w.G5};   // free once the sweep is done
+    double2 *H[4] = {work, work + F1, work + 2 * F1, work + 3 * F1};   // free once the sweep is done
     for (int nu = 0; nu < 4; nu++) k_lep_h<<<grid2, 128, 0, cx.s>>>(H[nu], mid + nu * F1, Uf(nu), nu, g);
     for (int mu = 0; mu < 4; mu++) {
       const double2 *o[3];
@@ -411,7 +466,7 @@ int smear_adjoint(const double2 *U, const double c[6], const double2 *mid, const
     nk += 8;
   }
   QLAUNCHN(nk);
-  return nk;
+  return sweep_terms(c, midN != nullptr, lepage_rep);
 }
 
 // outer products of sources [first, first + n) into mid (and midN)
@@ -444,7 +499,7 @@ void asqtad_force(QOP_info_t *info, GaugeT<T> *G, GaugeT<T> *F, const QOP_asqtad
   const bool naik = cf->naik != 0;
   double2 *mid = dalloc<double2>(naik ? 2 * F4 : F4), *D = dalloc<double2>(F4);
   dzero(D, sizeof(double2) * F4);
-  const SweepWork w{dalloc<double2>(F1), dalloc<double2>(F1), dalloc<double2>(F1), dalloc<double2>(F1)};
+  double2 *w = dalloc<double2>(SWEEP_FIELDS * F1);
   force_mids<T>(mid, naik ? mid + F4 : nullptr, x, eps, nsrc, -1.0);   // scale -1 (fnmat_p.c:497)
   const double co[6] = {cf->one_link, cf->three_staple, cf->five_staple, cf->seven_staple, cf->lepage, cf->naik};
   const int nk = smear_adjoint(U, co, mid, naik ? mid + F4 : nullptr, D, w);
@@ -459,7 +514,7 @@ void asqtad_force(QOP_info_t *info, GaugeT<T> *G, GaugeT<T> *F, const QOP_asqtad
   k_force_ta<T><<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(F->d, U, D, asvec ? -1.0 : -2.0, g);
   QLAUNCH();
   sync();
-  dfree(mid); dfree(D); dfree(w.S3); dfree(w.S5); dfree(w.G3); dfree(w.G5);
+  dfree(mid); dfree(D); dfree(w);
   if (own) dfree(U);
   if (info) {
     info->final_sec = wtime() - t0;
@@ -485,7 +540,7 @@ void hisq_force(QOP_info_t *info, HisqT<T> *h, GaugeT<T> *F, const QOP_hisq_coef
   double2 *D = dalloc<double2>(F4);
   dzero(GW, sizeof(double2) * F4);
   dzero(D, sizeof(double2) * F4);
-  const SweepWork w{dalloc<double2>(F1), dalloc<double2>(F1), dalloc<double2>(F1), dalloc<double2>(F1)};
+  double2 *w = dalloc<double2>(SWEEP_FIELDS * F1);
   int nterms = 0;
   for (int k = 0; k < cf->n_naiks; k++) nterms += n_orders[k];
   const double ca[6] = {cf->asqtad_one_link, cf->asqtad_three_staple, cf->asqtad_five_staple,
@@ -512,7 +567,7 @@ void hisq_force(QOP_info_t *info, HisqT<T> *h, GaugeT<T> *F, const QOP_hisq_coef
   k_force_ta<T><<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(F->d, U, D, 2.0, g);   // deriv = 2 D
   QLAUNCH();
   sync();
-  dfree(mid); dfree(GW); dfree(T1); dfree(D); dfree(w.S3); dfree(w.S5); dfree(w.G3); dfree(w.G5);
+  dfree(mid); dfree(GW); dfree(T1); dfree(D); dfree(w);
   if (oU) dfree(U);
   if (oV) dfree(V);
   if (oW) dfree(W);

@@ -9,54 +9,30 @@
 #include "fields.cuh"
 #include "reduce.cuh"
 #include "dslash.cuh"
-#include "mat3.cuh"
+#include "staple.cuh"
 #include <cmath>
 
 namespace qopb {
 
 
 // ---------------------------------------------------------------- staples
-// upper(x) = U_nu(x) [link(x+nu) U_nu(x+mu)^+]
-// lower(x) = [U_nu(y)^+ link(y)] U_nu(y+mu),  y = x - nu
-// SAVE: save = upper + lower, fl += coef save; else fl += coef upper; fl += coef lower
-template <bool SAVE>
-__global__ void k_staple(double2 *fl, double2 *save, const double2 *link, const double2 *Unu, int mu, int nu,
-                         double coef, Geom g) {
-  i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  const int p = (int)(s / g.Vh), i = (int)(s % g.Vh);
+// fl = c1 in + w sum_n staple(Y_n; n)  (staple.cuh; w 0: no staples)
+struct FatArgs {
+  const double2 *in, *Y[3];
+  double2 *fl;
+  double c1, w;
+};
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_fat(const __grid_constant__ FatArgs f, const __grid_constant__ StU U, int mu, Geom g) {
+  int grp, p, i;
+  if (!st_block(g, 1, grp, p, i)) return;
+  const StSite s = st_site(g, i, p);
+  const int r = threadIdx.y;
   const i64 Vh = g.Vh;
-  int x[4], y[4];
-  site_coords(g, i, p, x);
-  int pn, in_, pm, im, py, iy, pym, iym;
-  shifted(g, x, nu, 1, y); par_idx(g, y, pn, in_);
-  shifted(g, x, mu, 1, y); par_idx(g, y, pm, im);
-  int yy[4];
-  shifted(g, x, nu, -1, yy); par_idx(g, yy, py, iy);
-  shifted(g, yy, mu, 1, y); par_idx(g, y, pym, iym);
-  M3 t1 = mul_na(ld3(fptr(link, g, pn, in_), Vh), ld3(fptr(Unu, g, pm, im), Vh));
-  M3 up = mul(ld3(fptr(Unu, g, p, i), Vh), t1);
-  t1 = mul_an(ld3(fptr(Unu, g, py, iy), Vh), ld3(fptr(link, g, py, iy), Vh));
-  M3 lo = mul(t1, ld3(fptr(Unu, g, pym, iym), Vh));
-  double2 *F = fl + (i64)p * 9 * Vh + i;
-  if (SAVE) {
-    double2 *S = save + (i64)p * 9 * Vh + i;
+  double2 a[1][3] = {};
+  st_fat_row(g, s, f.in, f.Y, U, f.c1, f.w, mu, r, a);
+  double2 *o = st_at(f.fl, Vh, p, s.lex);
 #pragma unroll
-    for (int e = 0; e < 9; e++) {
-      double2 v = make_double2(up.e[e].x + lo.e[e].x, up.e[e].y + lo.e[e].y);
-      S[e * Vh] = v;
-      double2 f = F[e * Vh];
-      F[e * Vh] = make_double2(f.x + coef * v.x, f.y + coef * v.y);
-    }
-  } else {
-#pragma unroll
-    for (int e = 0; e < 9; e++) {
-      double2 f = F[e * Vh];
-      f.x += coef * up.e[e].x; f.y += coef * up.e[e].y;
-      f.x += coef * lo.e[e].x; f.y += coef * lo.e[e].y;
-      F[e * Vh] = f;
-    }
-  }
+  for (int c = 0; c < 3; c++) o[(3 * r + c) * Vh] = a[0][c];
 }
 
 __global__ void k_scale_field(double2 *d, const double2 *s, double c, i64 n) {
@@ -66,67 +42,72 @@ __global__ void k_scale_field(double2 *d, const double2 *s, double c, i64 n) {
   d[k] = make_double2(c * v.x, c * v.y);
 }
 
-// ll(x) = naik U(x) [U(x+mu) U(x+2mu)]
-__global__ void k_naik(double2 *ll, const double2 *U, int mu, double naik, Geom g) {
-  i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
-  if (s >= 2 * g.Vh) return;
-  const int p = (int)(s / g.Vh), i = (int)(s % g.Vh);
-  int x[4], y[4], p1, i1, p2, i2;
-  site_coords(g, i, p, x);
-  shifted(g, x, mu, 1, y); par_idx(g, y, p1, i1);
-  shifted(g, x, mu, 2, y); par_idx(g, y, p2, i2);
-  M3 t = mul(ld3(fptr(U, g, p1, i1), g.Vh), ld3(fptr(U, g, p2, i2), g.Vh));
-  M3 r = mul(ld3(fptr(U, g, p, i), g.Vh), t);
+// ll(x) = naik U(x) U(x+mu) U(x+2mu), the four directions as block groups
+struct NaikArgs {
+  double2 *ll[4];
+};
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_naik(const __grid_constant__ NaikArgs n, const __grid_constant__ StU U, double naik, Geom g) {
+  int mu, p, i;
+  if (!st_block(g, 4, mu, p, i)) return;
+  const StSite s = st_site(g, i, p);
+  const int r = threadIdx.y;
+  const i64 Vh = g.Vh;
+  double2 u[3], t[3], o[3];
+  st_row(st_at(U.d[mu], Vh, p, s.lex), Vh, r, u);
+  st_mul(u, st_at(U.d[mu], Vh, 1 - p, s.lex + st_step(g, s, mu, 1)), Vh, t);
+  st_mul(t, st_at(U.d[mu], Vh, p, s.lex + st_step(g, s, mu, 2)), Vh, o);
+  double2 *l = st_at(n.ll[mu], Vh, p, s.lex);
 #pragma unroll
-  for (int e = 0; e < 9; e++) { r.e[e].x *= naik; r.e[e].y *= naik; }
-  st3(ll + (i64)p * 9 * g.Vh + i, g.Vh, r);
-}
-
-static void staple(double2 *fl, double2 *save, const double2 *link, const double2 *Unu, int mu, int nu, double coef) {
-  const Geom &g = ctx().g;
-  int grid = grid_for(2 * g.Vh, 128);
-  if (save) k_staple<true><<<grid, 128, 0, ctx().s>>>(fl, save, link, Unu, mu, nu, coef, g);
-  else k_staple<false><<<grid, 128, 0, ctx().s>>>(fl, nullptr, link, Unu, mu, nu, coef, g);
-  QLAUNCH();
+  for (int c = 0; c < 3; c++) l[(3 * r + c) * Vh] = make_double2(naik * o[c].x, naik * o[c].y);
 }
 
 // make_imp_links (asqtad_dslash_p.c:458-633): gf, gfLong, fl, ll are
-// [4][2][9][Vh] FP64 fields; ll may be null (no Naik term)
+// [4][2][9][Vh] FP64 fields; ll may be null (no Naik term).  Per direction
+// three kernels (S_n, X_n, fat link; staple.cuh) instead of one per staple:
+// 12 staples and about 25 field passes where 18 staples took about 95.  The
+// latency of the L2 reads bounds them (24^3 x 48, HISQ: the whole call 9.4 ms
+// against 22.4 with one launch per staple; 12^4: 0.44 against 1.35 ms).
 static double make_imp_links(const QOP_asqtad_coeffs_t *cf, const double2 *gf, const double2 *gfLong, double2 *fl,
                              double2 *ll) {
   const Geom &g = ctx().g;
+  const cudaStream_t st = ctx().s;
   const i64 F = 18 * g.Vh;
   double c1 = cf->one_link, c3 = cf->three_staple, c5 = cf->five_staple, c7 = cf->seven_staple, cL = cf->lepage;
   c1 -= 6 * cL;
-  bool have5 = c5 != 0 || c7 != 0 || cL != 0;
-  bool have3 = c3 != 0 || have5;
-  double2 *stp = dalloc<double2>(F), *tmp = dalloc<double2>(F);
+  const bool have5 = c5 != 0 || c7 != 0 || cL != 0;
+  const bool have3 = c3 != 0 || have5;
+  const StU U{{gf, gf + F, gf + 2 * F, gf + 3 * F}};
+  double2 *work = have5 ? dalloc<double2>(6 * F) : nullptr;   // S_n and X_n of one direction
   for (int dir = 0; dir < 4; dir++) {
-    k_scale_field<<<grid_for(F, 256), 256, 0, ctx().s>>>(fl + dir * F, gf + dir * F, c1, F);
-    QLAUNCH();
-    if (!have3) continue;
-    for (int nu = 0; nu < 4; nu++) {
-      if (nu == dir) continue;
-      staple(fl + dir * F, stp, gf + dir * F, gf + nu * F, dir, nu, c3);
-      if (cL != 0) staple(fl + dir * F, nullptr, stp, gf + nu * F, dir, nu, cL);
-      if (c5 != 0 || c7 != 0) {
-        for (int rho = 0; rho < 4; rho++) {
-          if (rho == dir || rho == nu) continue;
-          staple(fl + dir * F, tmp, stp, gf + rho * F, dir, rho, c5);
-          if (c7 != 0)
-            for (int sig = 0; sig < 4; sig++)
-              if (sig != dir && sig != nu && sig != rho) staple(fl + dir * F, nullptr, tmp, gf + sig * F, dir, sig, c7);
-        }
-      }
+    const double2 *in = gf + dir * F;
+    if (!have3) {
+      k_scale_field<<<grid_for(F, 256), 256, 0, st>>>(fl + dir * F, in, c1, F);
+      QLAUNCH();
+      continue;
     }
+    FatArgs fa{in, {in, in, in}, fl + dir * F, c1, c3};
+    if (have5) {
+      StChain<1> ch;
+      ch.in[0] = in;
+      ch.c3[0] = c3;
+      for (int j = 0; j < 3; j++) {
+        ch.S[0][j] = work + j * F;
+        fa.Y[j] = ch.X[0][j] = work + (3 + j) * F;
+      }
+      fa.w = 1.0;
+      k_chain_s<1><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, U, dir, g);
+      k_chain_x<1><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, U, StCoef{cL, c5, c7}, dir, g);
+      QLAUNCHN(2);
+    }
+    k_fat<<<st_grid(g, 1), st_threads(), 0, st>>>(fa, U, dir, g);
+    QLAUNCH();
   }
   if (ll) {
-    for (int dir = 0; dir < 4; dir++) {
-      k_naik<<<grid_for(2 * g.Vh, 128), 128, 0, ctx().s>>>(ll + dir * F, gfLong + dir * F, dir, cf->naik, g);
-      QLAUNCH();
-    }
+    const StU UL{{gfLong, gfLong + F, gfLong + 2 * F, gfLong + 3 * F}};
+    k_naik<<<st_grid(g, 4), st_threads(), 0, st>>>(NaikArgs{{ll, ll + F, ll + 2 * F, ll + 3 * F}}, UL, cf->naik, g);
+    QLAUNCH();
   }
-  dfree(stp); dfree(tmp);
+  dfree(work);
   return (have3 || cf->naik != 0) ? 61632.0 * (double)g.V : 0.0;
 }
 
