@@ -249,6 +249,7 @@ template <typename T> struct Blas {
 template <typename TD, typename TS> void convert(c2<TD> *d, const c2<TS> *s, Range r);
 
 // ---------------------------------------------------------------- dslash (dslash.cu)
+struct CgState;   // cg.cuh
 template <typename T> struct Dslash {
   // reference semantics of QOP_asqtad_dslash_qdp (lib/asqtad_dslash_p.c:1048-1092)
   static void apply(FlaT<T> *f, double mass, c2<T> *out, const c2<T> *in, int eo_out, int eo_in);
@@ -260,6 +261,11 @@ template <typename T> struct Dslash {
   // tmp receives D_oe in on the opposite parity; returns |tmp|^2 + m^2 |in|^2
   static double ddagd(FlaT<T> *f, double mass, c2<T> *out, const c2<T> *in, int eo,
                       c2<T> *tmp, bool want_norm);
+  // the two hops of one iteration of a device-driven CG (cg.cuh): out = A in
+  // and the step length in *st; dot: from <in, out>, else from |D in|^2 +
+  // m^2 |in|^2; first: an ordinary launch, else a dependent of the launch ahead
+  static void cg_hops(FlaT<T> *f, double mass, c2<T> *out, const c2<T> *in, int eo, c2<T> *tmp, CgState *st, bool dot,
+                      bool first);
   // the same operator with caller-provided scratch: tmp_block is one parity
   // block ([3][Vh]), part/count/res the reduction partials, ticket and the
   // two sums; launches only, no allocation and no synchronisation
