@@ -8,6 +8,8 @@
 #include "solvers.cuh"
 #include <memory>
 #include "fields.cuh"
+#include "cg.cuh"
+#include <algorithm>
 #include <vector>
 #include <cmath>
 #include <type_traits>
@@ -43,6 +45,7 @@ void cg(LinOp<T> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *ra, c2<T> *out, cons
   Tmp<T> r, Mp;
   double rsqstop = ra->rsqmin * insq, rsq = 0, oldrsq = 0, relnorm = 1;
   log0(QOP_VERB_LOW, "CG: rsqmin = %g relmin = %g\nCG: rsqstop = %g\n", ra->rsqmin, ra->relmin, rsqstop);
+  const bool dev = cg_on_device(eo) && !(ra->relmin > 0);   // a relative norm is read every iteration
   while (true) {
     if (total == 0 || iteration >= restart_it || total >= max_it || rsq < rsqstop || relnorm < ra->relmin) {
       if (total >= max_it || nrestart >= max_restarts) break;
@@ -60,6 +63,21 @@ void cg(LinOp<T> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *ra, c2<T> *out, cons
     } else {
       double b = rsq / oldrsq;
       B::xpay(p, r, b, q);
+    }
+    if (dev) {   // every iteration up to the next restart or the end
+      CgState s{};
+      s.rsq = rsq;
+      s.fac = 1;
+      s.stop = rsqstop;
+      s.left = std::max(1, std::min(restart_it - iteration, max_it - total));
+      cg_run<T>(L, out, r, p, Mp, eo, true, s);
+      iteration += s.done; total += s.done;
+      oldrsq = s.oldrsq;
+      rsq = s.rsq;
+      if (s.flag == CG_EVENT) continue;
+      iteration++; total++;
+      need_finite(s.pkp, "CG: <p, A p>");
+      break;
     }
     oldrsq = rsq;
     L.d2(Mp, p);
@@ -116,15 +134,35 @@ void cgms(LinOp<T> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t **ra, const double 
   const int rsqCheckInterval = 100, relCheckInterval = 100;
   int nextRsqCheck = rsqCheckInterval, nextRelCheck = relCheckInterval;
   B::copy(ry, in, q);
+  const bool dev = ns == 1 && cg_on_device(eo) && !(relstop > 0);
   while (true) {
-    oldrsq = rsq;
-    double pkp = L.d2n(Mp, p);
-    iteration++;
-    need_finite(pkp, "CGMS: <p, A p>");
-    if (pkp <= 0) break;
-    b[imin] = rsq / pkp;
-    rsq = B::cg_update(out[imin], r, b[imin], p, Mp, q);
-    zn[imin] = 1;
+    if (dev) {   // every iteration up to the next check of the true residual or the end
+      CgState s{};
+      s.rsq = rsq;
+      s.fac = trueRsqFac;
+      s.stop = rsqstop;
+      s.left = std::max(1, std::min(std::min(ia->restart, ia->max_iter), nextRsqCheck) - iteration);
+      cg_run<T>(L, out[imin], r, p, Mp, eo, false, s);
+      iteration += s.done;
+      oldrsq = s.oldrsq;
+      rsq = s.rsq;
+      b[imin] = s.a;
+      zn[imin] = 1;
+      if (s.flag != CG_EVENT) {
+        iteration++;
+        need_finite(s.pkp, "CGMS: <p, A p>");
+        break;
+      }
+    } else {
+      oldrsq = rsq;
+      double pkp = L.d2n(Mp, p);
+      iteration++;
+      need_finite(pkp, "CGMS: <p, A p>");
+      if (pkp <= 0) break;
+      b[imin] = rsq / pkp;
+      rsq = B::cg_update(out[imin], r, b[imin], p, Mp, q);
+      zn[imin] = 1;
+    }
     for (int i = 0; i < ns; i++) {
       if (i == imin) continue;
       zn[i] = z[i] * zo[i] * bo[imin];
