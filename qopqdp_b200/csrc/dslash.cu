@@ -73,7 +73,7 @@ __device__ __forceinline__ void hop_mul(c2<T> (&a)[3], const c2<T> (&U)[9], c2<T
 // warps, which load their links before they wait for the kernel ahead (links
 // are never written by it: the first kernel of a dependent chain is an
 // ordinary launch), so a hop costs one round trip to L2 instead of one per
-// slot; the partial sums meet in shared memory in slot order.
+// slot; the partial sums meet in shared memory and are added in FP64.
 // BOTH: both parities in one launch, site blocks of the two parities next to
 // each other, and every link read as a forward link: a backward slot takes
 // the neighbour's forward link, which the neighbour's own block has brought
@@ -181,9 +181,15 @@ k_hop(c2<T> *__restrict__ out, const c2<T> *__restrict__ src, const c2<T> *__res
     live = live && w == 0;
     if (live) {
 #pragma unroll
-      for (int q = 0; q < SPLIT - 1; q++)
+      for (int r = 0; r < 3; r++) {   // one rounding for the whole sum
+        double re = a[r].x, im = a[r].y;
 #pragma unroll
-        for (int r = 0; r < 3; r++) a[r] = cadd<T>(a[r], sh[q][r][t]);
+        for (int q = 0; q < SPLIT - 1; q++) {
+          re += sh[q][r][t].x;
+          im += sh[q][r][t].y;
+        }
+        a[r] = mk<T>((T)re, (T)im);
+      }
     }
   }
   double racc[1] = {0.0};
@@ -283,7 +289,7 @@ template <typename T> constexpr int hop_split() { return sizeof(T) == 4 ? 4 : 8;
 // 32800 26 / 25 and 37 / 34.
 template <typename T> static bool use_split(i64 Vh, bool both) {
   if (both) return Vh <= 20000;
-  return sizeof(T) == 4 || Vh <= 210000;
+  return Vh <= (sizeof(T) == 4 ? 130000 : 210000);
 }
 
 // x1 coordinates per tile of a two-parity hop: the forward links of the four
