@@ -28,6 +28,7 @@
 #include "fields.cuh"
 #include "mixed.cuh"
 #include "dd.cuh"
+#include "pdl.cuh"
 #include <algorithm>
 #include <array>
 #include <map>
@@ -138,31 +139,6 @@ k_mix_p(typename Sp::elem *__restrict__ p, const typename Sp::elem *__restrict__
 #pragma unroll
   for (int c = 0; c < 3; c++) pv[c] = make_float2(fmaf(be, pv[c].x, rv[c].x), fmaf(be, pv[c].y, rv[c].y));
   Sp::store(p, i, Vh, pv);
-}
-
-// Programmatic dependent launch (option pdl): a kernel launched with the
-// attribute may be scheduled while the kernel ahead of it in the stream
-// drains; griddepcontrol.wait holds it until that kernel has completed and
-// its memory is visible.  Without the attribute the wait returns at once.
-__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
-
-template <typename... KArgs, typename... Args>
-static void launch_k(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
-  if (!pdl) {
-    k<<<grid, block, 0, s>>>(args...);
-    return;
-  }
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = grid;
-  cfg.blockDim = block;
-  cfg.dynamicSmemBytes = 0;
-  cfg.stream = s;
-  cudaLaunchAttribute at[1];
-  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  at[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = at;
-  cfg.numAttrs = 1;
-  QCHECK(cudaLaunchKernelEx(&cfg, k, args...));
 }
 
 // x += alpha p, r -= alpha Ap and p = r + beta p in one pass (fused update:
@@ -1032,6 +1008,106 @@ k_mix_hop_q16r(uint4 *__restrict__ out, const uint4 *__restrict__ src, const uns
 }
 
 
+// The fused iteration's hops on small lattices: 64 sites per block and four
+// warps' worth of threads per 32 sites, each holding the slots of one
+// direction, so that a hop is one round trip to L2 for the links and one for
+// the neighbours where a thread per site makes four of each, and four times
+// as many warps cover them.  The links (never written by the kernel ahead:
+// the first kernel of a chunk is an ordinary launch) are requested before the
+// wait for it; the row sums of the four parts meet in shared memory in slot
+// order.  KIND 1 and 3.
+constexpr int Q16S_SITES = 64;
+template <int NL, int KIND, bool RECON>
+__global__ void __launch_bounds__(4 * Q16S_SITES)
+k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned char *__restrict__ lk,
+               const uint4 *__restrict__ same, Geom g, NbrGeom ng, int p, MixState *st, double *part,
+               unsigned *count, float c_long, const uint4 *__restrict__ rres, int seq) {
+  constexpr int NS = NL / 4;
+  const int t = threadIdx.x % Q16S_SITES, w = threadIdx.x / Q16S_SITES;   // w: uniform over a warp, the direction
+  const i64 Vh = g.Vh;
+  const int i = blockIdx.x * Q16S_SITES + t, tb = i % QB;   // the link blocks are padded to QB sites
+  const bool live = i < Vh;
+  const unsigned char *gl = lk + (size_t)(i / QB) * q16_block_bytes(NL, RECON) + q16_slot_off(w * NS, RECON);
+  uint4 ua[NS], ub[NS];
+  uint2 uc[NS];
+  int j[NS];
+  int x[4];
+  site_coords(g, live ? i : 0, p, x);
+  const int lex = ((x[0] * g.L[1] + x[1]) * g.L[2] + x[2]) * g.L[3] + x[3];
+#pragma unroll
+  for (int s = 0; s < NS; s++) {
+    const unsigned char *ls = gl + q16_slot_off(s, RECON);
+    ua[s] = reinterpret_cast<const uint4 *>(ls)[tb];
+    if (RECON && (s & 1)) {
+      const uint2 v = reinterpret_cast<const uint2 *>(ls + 16 * QB)[tb];
+      ub[s] = make_uint4(v.x, v.y, 0u, 0u);
+      uc[s] = make_uint2(__float_as_uint(reinterpret_cast<const float *>(ls + 24 * QB)[tb]), 0u);
+    } else {
+      ub[s] = reinterpret_cast<const uint4 *>(ls + 16 * QB)[tb];
+      uc[s] = reinterpret_cast<const uint2 *>(ls + 32 * QB)[tb];
+    }
+    j[s] = nbr_sel(ng, x[0], x[1], x[2], x[3], lex, w, slot_disp<NL>(s));
+  }
+  pdl_wait();
+  if (st->flag) return;
+  uint4 nb[NS], sraw = make_uint4(0, 0, 0, 0), rraw = sraw;
+#pragma unroll
+  for (int s = 0; s < NS; s++) nb[s] = src[j[s]];
+  if (KIND == 3 && w == 0 && live) {
+    sraw = same[i];
+    rraw = rres[i];
+  }
+  float2 a[3], pt[3], ps[3];
+#pragma unroll
+  for (int r = 0; r < 3; r++) pt[r] = ps[r] = make_float2(0.f, 0.f);
+#pragma unroll
+  for (int s = 0; s < NS; s++) {
+    if (RECON && (s & 1))
+      q16_slot_recon_pk(ua[s], make_uint2(ub[s].x, ub[s].y), __uint_as_float(uc[s].x), nb[s], c_long, pt, ps);
+    else
+      q16_slot_pk(ua[s], ub[s], uc[s], nb[s], pt, ps);
+  }
+  q16_pk_rows(pt, ps, a);
+  __shared__ float2 sh[3][3][Q16S_SITES];
+  if (w > 0) {
+#pragma unroll
+    for (int r = 0; r < 3; r++) sh[w - 1][r][t] = a[r];
+  }
+  __syncthreads();
+  double acc[KIND == 3 ? 3 : 1];
+#pragma unroll
+  for (int k = 0; k < (KIND == 3 ? 3 : 1); k++) acc[k] = 0.0;
+  if (w == 0 && live) {
+#pragma unroll
+    for (int q = 0; q < 3; q++)
+#pragma unroll
+      for (int r = 0; r < 3; r++) a[r] = cadd<float>(a[r], sh[q][r][t]);
+    if constexpr (KIND == 3) q16_epilogue3(out + i, &sraw, &rraw, 0, Vh, (float)st->m2, a, acc);
+    else acc[0] = q16_epilogue<1>(out, nullptr, i, Vh, 0.f, a);
+  }
+  if constexpr (KIND == 3) q16_finish3<false>(acc, part, count, st, seq);
+  else q16_finish<1>(acc, part, count, st);
+}
+
+// The split hops take the default variant's place between the smallest size
+// that was timed and the one where HBM and issue take over from latency (ms per
+// solve, split / general: 8^4 13.3 / 15.7, 12^4 14.6 / 17.3, 16^4 20.1 / 22.2,
+// 16^3x32 30.5 / 28.8, 20^4 36.5 / 31.5).
+static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh >= 2048 && Vh <= 32768; }
+
+template <int KIND>
+static void launch_q16_small(int nl, bool recon, float c_long, uint4 *out, const uint4 *src, const unsigned char *lk,
+                             const uint4 *same, const Geom &g, const NbrGeom &ng, int par, MixState *st,
+                             const uint4 *rres, int seq, bool pdl) {
+  Context &c = ctx();
+  const int grid = grid_for(g.Vh, Q16S_SITES);
+#define Q16S_ARGS grid, 4 * Q16S_SITES, c.s, out, src, lk, same, g, ng, par, st, c.d_part, c.d_count, c_long, rres, seq
+  if (nl != 16) launch_k(pdl, k_mix_hop_q16s<8, KIND, false>, Q16S_ARGS);
+  else if (recon) launch_k(pdl, k_mix_hop_q16s<16, KIND, true>, Q16S_ARGS);
+  else launch_k(pdl, k_mix_hop_q16s<16, KIND, false>, Q16S_ARGS);
+#undef Q16S_ARGS
+}
+
 static std::map<void *, SloppyLinks *> g_sloppy;
 
 void sloppy_invalidate(void *fla_any) {
@@ -1441,6 +1517,8 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
   const bool fuse = q16v && c.opt.fuse_update && hk >= 20;
   // the three kernels of the fused iteration as programmatic dependents
   const bool pdl = fuse && c.opt.pdl;
+  // the default hop on a small lattice (the numbered variants keep their shapes)
+  const bool small = fuse && !dd_active() && use_q16_small(Vh);
   int seq = 0;
   // a decomposed lattice: halos before each hop, the reductions summed over
   // the processes before the scalars (the fused int16 iteration only)
@@ -1482,7 +1560,13 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
         ProfScope ps1(hname, hop_bytes);
         if constexpr (std::is_same<Lk, LkQ16B>::value) {
           const unsigned char *lq = (const unsigned char *)lk_q.a;
-          launch_q16<1>(hk, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst, pdl);
+          if constexpr (q16v) {
+            if (small)
+              launch_q16_small<1>(nl, recon, c_long, ts, ps, lq, nullptr, g, ng, q, dst, nullptr, 0, pdl && k > 0);
+            else launch_q16<1>(hk, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst, pdl);
+          } else {
+            launch_q16<1>(hk, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst, pdl);
+          }
         } else {
           if (nl == 16) k_mix_hop<Sp, Lk, 16, 1><<<gridh, 128, 0, c.s>>>(ts, ps, lk_q, nullptr, g, q, dst, c.d_part, c.d_count);
           else k_mix_hop<Sp, Lk, 8, 1><<<gridh, 128, 0, c.s>>>(ts, ps, lk_q, nullptr, g, q, dst, c.d_part, c.d_count);
@@ -1493,7 +1577,9 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
         ProfScope ps2(fuse ? hname3 : hname, hop_bytes + (double)Vh * Sp::site_bytes * (fuse ? 2 : 1));
         if constexpr (q16v) {
           const unsigned char *lp = (const unsigned char *)lk_p.a;
-          if (fuse) launch_q16_fused(hk, nl, recon, c_long, gridq, Aps, ts, lp, ps, g, ng, p, dst, rs, ++seq, pdl);
+          if (small)
+            launch_q16_small<3>(nl, recon, c_long, Aps, ts, lp, ps, g, ng, p, dst, rs, ++seq, pdl);
+          else if (fuse) launch_q16_fused(hk, nl, recon, c_long, gridq, Aps, ts, lp, ps, g, ng, p, dst, rs, ++seq, pdl);
           else launch_q16<2>(hk, nl, recon, c_long, gridq, Aps, ts, lp, ps, g, ng, p, dst);
         } else if constexpr (std::is_same<Lk, LkQ16B>::value) {
           const unsigned char *lp = (const unsigned char *)lk_p.a;
@@ -1813,10 +1899,18 @@ extern "C" int QOPB_D3_sloppy_ddagd(QOP_info_t *info, QOP_D3_FermionLinksAsqtad 
     QLAUNCH();
     const bool recon = sl->recon != 0;
     const float c_long = (float)sl->c_long;
-    launch_q16<1>(variant, sl->nl, recon, c_long, gridq, t16, p16, (const unsigned char *)lk_q.a, nullptr, g, ng, q,
-                  dst);
+    const bool small = variant == 25 && kind2 == 3 && use_q16_small(Vh);   // as the solver chooses
+    if (small)
+      launch_q16_small<1>(sl->nl, recon, c_long, t16, p16, (const unsigned char *)lk_q.a, nullptr, g, ng, q, dst,
+                          nullptr, 0, false);
+    else
+      launch_q16<1>(variant, sl->nl, recon, c_long, gridq, t16, p16, (const unsigned char *)lk_q.a, nullptr, g, ng, q,
+                    dst);
     QLAUNCH();
-    if (kind2 == 3)
+    if (small)
+      launch_q16_small<3>(sl->nl, recon, c_long, a16, t16, (const unsigned char *)lk_p.a, p16, g, ng, p, dst, p16, 1,
+                          true);
+    else if (kind2 == 3)
       launch_q16_fused(variant, sl->nl, recon, c_long, gridq, a16, t16, (const unsigned char *)lk_p.a, p16, g, ng, p,
                        dst, p16, 1);
     else
