@@ -29,6 +29,7 @@
 #include "fields.cuh"
 #include "mixed.cuh"
 #include "bmma.cuh"
+#include "pdl.cuh"
 #include <algorithm>
 #include <array>
 #include <map>
@@ -233,11 +234,198 @@ k_bhop(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned ch
   }
 }
 
-// x_j += alpha_j p_j, r_j -= alpha_j Ap_j, |r_j|^2: blockIdx.y = system
+// slots of a launch: the systems still running when the chunk was launched
+struct BList {
+  int n, s[BATCH_MAX];
+};
+
+// The batched hop with the slots of a launch taken from a list, spread evenly
+// over groups of up to 2 BP systems per thread, so that a launch with few
+// systems left has few groups.  The two lanes of every packed FP32 operation
+// are two systems, so the row sums of a system take 6 registers (12 with the
+// real and imaginary part in the lanes) and 8 systems share one decode of a
+// link.  Per pair of systems and slot: two 16-byte loads, 12 byte permutes,
+// 6 packed adds and 9 packed multiplies for the decode and 36 packed FMAs.
+// Latency and instruction issue bound it (a packed FMA takes two cycles of the
+// FP32 pipe; with the parts of one system in the lanes it issued at 51 % with
+// 16 warps per SM).  us per hop by running systems at 24^3x48 (variants 1 / 7
+// before): 16 242 (270), 13 256 (257), 12 215 (242), 9 201 (206), 7 150 (168),
+// 6 125 (166), 4 96 (139), 3 94 (134), 2 66 (127); 32^4, 16 sources, m 0.05:
+// the call 857 ms (1016).  A ring of cp.async stages in shared memory gained
+// less (252 us with 16) than it cost to order its refills.  A lane without a system of its own repeats the group's first
+// one and stores nothing.
+template <int NL, int KIND, bool RECON, int BP, int MINB>
+__global__ void __launch_bounds__(QB, MINB)
+k_bhop_pair(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned char *__restrict__ lk,
+            const uint4 *__restrict__ same, Geom g, NbrGeom ng, int p, MixState *st, const __grid_constant__ BList bl,
+            int ngrp, double *part, unsigned *count, float c_long) {
+  constexpr int BG = 2 * BP;
+  const int grp = blockIdx.x % ngrp, sb = blockIdx.x / ngrp, nsb = gridDim.x / ngrp;
+  const int tid = threadIdx.x;
+  const i64 Vh = g.Vh;
+  const int i = sb * QB + tid;
+  // group grp holds list entries [lo, hi)
+  const int per = bl.n / ngrp, more = bl.n - per * ngrp;
+  const int lo = grp * per + min(grp, more), hi = lo + per + (grp < more ? 1 : 0);
+  pdl_wait();
+  unsigned act = 0;   // bit b: entry lo + b exists and runs
+#pragma unroll
+  for (int b = 0; b < BG; b++)
+    if (lo + b < hi && st[bl.s[lo + b]].flag == 0) act |= 1u << b;
+  if (!act) return;   // uniform over the group: no block of it reduces
+  int sys[BG];
+#pragma unroll
+  for (int b = 0; b < BG; b++) sys[b] = bl.s[lo + b < hi ? lo + b : lo];
+  double acc[BG];
+#pragma unroll
+  for (int b = 0; b < BG; b++) acc[b] = 0.0;
+  if (i < Vh) {
+    int x[4];
+    site_coords(g, i, p, x);
+    const int x0 = x[0], x1 = x[1], x2 = x[2], x3 = x[3];
+    const int lex = ((x0 * g.L[1] + x1) * g.L[2] + x2) * g.L[3] + x3;
+    float2 re[BP][3], im[BP][3];   // row sums: (system 2q, system 2q + 1)
+#pragma unroll
+    for (int q = 0; q < BP; q++)
+#pragma unroll
+      for (int r = 0; r < 3; r++) re[q][r] = im[q][r] = make_float2(0.f, 0.f);
+    int off[BG];   // slots x Vh fits: at 88 bytes a slot and site an engine would pass 180 GB first
+#pragma unroll
+    for (int b = 0; b < BG; b++) off[b] = sys[b] * (int)Vh;
+    const unsigned char *gl = lk + (size_t)sb * q16_block_bytes(NL, RECON);
+#pragma unroll 2
+    for (int k = 0; k < NL; k++) {
+      const unsigned char *ls = gl + q16_slot_off(k, RECON);
+      const int nbi = nbr_sel(ng, x0, x1, x2, x3, lex, slot_mu<NL>(k), slot_disp<NL>(k));
+      uint4 nb[BG];
+#pragma unroll
+      for (int b = 0; b < BG; b++) nb[b] = src[off[b] + nbi];
+      float2 U[9];
+      float sl;
+      if (RECON && (k & 1)) {
+        const uint4 ua = __ldcs(reinterpret_cast<const uint4 *>(ls) + tid);
+        const uint2 ub = __ldcs(reinterpret_cast<const uint2 *>(ls + 16 * QB) + tid);
+        const float ph = __ldcs(reinterpret_cast<const float *>(ls + 24 * QB) + tid);
+        sl = q16_link_recon_pk(ua, ub, ph, c_long, U);
+      } else {
+        const uint4 ua = __ldcs(reinterpret_cast<const uint4 *>(ls) + tid);
+        const uint4 ub = __ldcs(reinterpret_cast<const uint4 *>(ls + 16 * QB) + tid);
+        const uint2 uc = __ldcs(reinterpret_cast<const uint2 *>(ls + 32 * QB) + tid);
+        sl = q16_link_pk(ua, ub, uc, U);
+      }
+      float2 ur[9], ui[9];
+#pragma unroll
+      for (int e = 0; e < 9; e++) {
+        ur[e] = make_float2(U[e].x, U[e].x);
+        ui[e] = make_float2(U[e].y, U[e].y);
+      }
+      sl *= 1.0f / 32767.0f;
+#pragma unroll
+      for (int q = 0; q < BP; q++) {
+        const uint4 na = nb[2 * q], nc = nb[2 * q + 1];
+        const float2 s2 = __fmul2_rn(make_float2(sl, sl), make_float2(__uint_as_float(na.w), __uint_as_float(nc.w)));
+        const float2 m2 = make_float2(-s2.x, -s2.y);
+        const unsigned wa[3] = {na.x, na.y, na.z}, wc[3] = {nc.x, nc.y, nc.z};
+        float2 vr[3], vi[3], vm[3];   // Re v, Im v, -Im v of the two systems
+#pragma unroll
+        for (int c = 0; c < 3; c++) {
+          const float2 off = make_float2(-8421376.0f, -8421376.0f);
+          const float2 r = __fadd2_rn(make_float2(__int_as_float(__byte_perm(wa[c], 0x4B000000u, 0x7610)),
+                                                  __int_as_float(__byte_perm(wc[c], 0x4B000000u, 0x7610))), off);
+          const float2 j = __fadd2_rn(make_float2(__int_as_float(__byte_perm(wa[c], 0x4B000000u, 0x7632)),
+                                                  __int_as_float(__byte_perm(wc[c], 0x4B000000u, 0x7632))), off);
+          vr[c] = __fmul2_rn(r, s2);
+          vi[c] = __fmul2_rn(j, s2);
+          vm[c] = __fmul2_rn(j, m2);
+        }
+#pragma unroll
+        for (int r = 0; r < 3; r++)
+#pragma unroll
+          for (int c = 0; c < 3; c++) {
+            re[q][r] = __ffma2_rn(ur[3 * r + c], vr[c], re[q][r]);
+            im[q][r] = __ffma2_rn(ur[3 * r + c], vi[c], im[q][r]);
+            re[q][r] = __ffma2_rn(ui[3 * r + c], vm[c], re[q][r]);
+            im[q][r] = __ffma2_rn(ui[3 * r + c], vr[c], im[q][r]);
+          }
+      }
+    }
+#pragma unroll
+    for (int b = 0; b < BG; b++) {
+      if (!(act >> b & 1)) continue;
+      const i64 o = (i64)sys[b] * Vh;
+      const int q = b / 2;
+      float2 a[3];
+#pragma unroll
+      for (int r = 0; r < 3; r++)
+        a[r] = b & 1 ? make_float2(re[q][r].y, im[q][r].y) : make_float2(re[q][r].x, im[q][r].x);
+      if (KIND == 1) {
+        acc[b] = (double)a[0].x * a[0].x + (double)a[0].y * a[0].y + (double)a[1].x * a[1].x +
+                 (double)a[1].y * a[1].y + (double)a[2].x * a[2].x + (double)a[2].y * a[2].y;
+        SpQ16::store(out + o, i, Vh, a);
+      } else {
+        const float m2 = (float)st[sys[b]].m2;
+        float2 sv[3];
+        SpQ16::load(same + o, i, Vh, sv);
+#pragma unroll
+        for (int c = 0; c < 3; c++) a[c] = make_float2(m2 * sv[c].x - a[c].x, m2 * sv[c].y - a[c].y);
+        SpQ16::store(out + o, i, Vh, a);
+        acc[b] = (double)sv[0].x * sv[0].x + (double)sv[0].y * sv[0].y + (double)sv[1].x * sv[1].x +
+                 (double)sv[1].y * sv[1].y + (double)sv[2].x * sv[2].x + (double)sv[2].y * sv[2].y;
+      }
+    }
+  }
+  __shared__ double res[BG];
+  if (group_sum<BG>(acc, part + (size_t)grp * nsb * BG, count + grp, res, sb, nsb)) {
+#pragma unroll
+    for (int b = 0; b < BG; b++) {
+      if (!(act >> b & 1)) continue;
+      MixState *s = st + sys[b];
+      if (KIND == 1) {
+        s->dp2 = res[b];
+      } else {
+        const double pAp = s->dp2 + s->m2 * res[b];   // <p, A p> = |D p|^2 + m^2 |p|^2
+        if (!(pAp > 0)) s->flag = MIX_BREAK;
+        else s->alpha = s->rsq / pAp;
+      }
+    }
+  }
+}
+
+// groups for n running systems: up to 8 in one, 9-12 in three of at most 4,
+// 13-16 in two of at most 8 (us per hop at 24^3x48: 12 systems 215 in three
+// groups, 254 in two of 6; 7 systems 150 in one, 162 in two; 16 systems 242 in
+// two, 245 in four, and at 32^4 885 against 925 ms per call)
+static int bhop_groups(int n) { return n <= 8 ? 1 : n <= 12 ? 3 : 2; }
+
+template <int KIND>
+static void launch_bhop_list(bool pdl, int nl, bool recon, int nsb, uint4 *out, const uint4 *src,
+                             const unsigned char *lk, const uint4 *same, const Geom &g, const NbrGeom &ng, int par,
+                             MixState *st, const BList &bl, double *part, unsigned *count, float c_long) {
+  Context &c = ctx();
+  const int ngrp = bhop_groups(bl.n), bp = ((bl.n + ngrp - 1) / ngrp + 1) / 2;
+#define BL_ARGS ngrp *nsb, QB, c.s, out, src, lk, same, g, ng, par, st, bl, ngrp, part, count, c_long
+#define BL_CALL(B, M)                                                              \
+  do {                                                                             \
+    if (nl != 16) launch_k(pdl, k_bhop_pair<8, KIND, false, B, M>, BL_ARGS);       \
+    else if (recon) launch_k(pdl, k_bhop_pair<16, KIND, true, B, M>, BL_ARGS);     \
+    else launch_k(pdl, k_bhop_pair<16, KIND, false, B, M>, BL_ARGS);               \
+  } while (0)
+  switch (bp) {
+    case 1: BL_CALL(1, 6); break;
+    case 2: BL_CALL(2, 5); break;
+    case 3: BL_CALL(3, 4); break;
+    default: BL_CALL(4, 4); break;
+  }
+#undef BL_CALL
+#undef BL_ARGS
+}
+
+// x_j += alpha_j p_j, r_j -= alpha_j Ap_j, |r_j|^2: blockIdx.y = list entry
 __global__ void __launch_bounds__(256)
 k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *__restrict__ p, const uint4 *__restrict__ Ap,
-          i64 Vh, MixState *st, double *part, unsigned *count) {
-  const int j = blockIdx.y;
+          i64 Vh, MixState *st, const __grid_constant__ BList bl, double *part, unsigned *count) {
+  pdl_wait();
+  const int j = bl.s[blockIdx.y];
   MixState *s = st + j;
   if (s->flag) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -263,7 +451,7 @@ k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *__restric
     acc1[0] = (double)rv[0].x * rv[0].x + (double)rv[0].y * rv[0].y + (double)rv[1].x * rv[1].x +
               (double)rv[1].y * rv[1].y + (double)rv[2].x * rv[2].x + (double)rv[2].y * rv[2].y;
   }
-  if (grid_sum<1>(acc1, part + (size_t)j * gridDim.x, count + j, &s->red)) {
+  if (grid_sum<1>(acc1, part + (size_t)blockIdx.y * gridDim.x, count + blockIdx.y, &s->red)) {
     const double rn = s->red;
     s->iter += 1;
     s->rsq_old = s->rsq;
@@ -274,10 +462,12 @@ k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *__restric
   }
 }
 
-// p_j = r_j + beta_j p_j: blockIdx.y = system
+// p_j = r_j + beta_j p_j: blockIdx.y = list entry
 __global__ void __launch_bounds__(256)
-k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState *st) {
-  const int j = blockIdx.y;
+k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState *st,
+     const __grid_constant__ BList bl) {
+  pdl_wait();
+  const int j = bl.s[blockIdx.y];
   if (st[j].flag) return;
   const int i = blockIdx.x * blockDim.x + threadIdx.x;
   if (i >= Vh) return;
@@ -294,7 +484,7 @@ k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState 
 // batched hop variants (option batch_kernel): systems per thread, the
 // register cap (resident blocks per SM) and the slot unrolling.  At 32^4
 // with 16 systems a hop takes 531 us with variant 7 (8 systems per thread,
-// 3 blocks per SM, slot loop unrolled by 2; the default), 557-580 us with
+// 3 blocks per SM, slot loop unrolled by 2), 557-580 us with
 // 1, 6, 9, 10, 605-679 us with 0, 2, 3, 5, 622 us with 8 and 705-1074 us
 // with 11 and 4 (16 / 8 systems, fully unrolled: ~240 registers).  The
 // kernel issues ~60-90 instructions per system and slot at ~55% issue
@@ -610,10 +800,7 @@ void BatchEngine::launch() {
   const float c_long = (float)sl->c_long;
   const int nsb = e.nsb, gridv = e.gridv;
   QCHECK(cudaMemcpyAsync(e.dst, e.h, sizeof(MixState) * n, cudaMemcpyHostToDevice, c.s));
-  // by default 8 systems per thread when they fill whole groups of 8 (16
-  // sources at 32^4: 531 us per hop against 574 with 4), else 4 (12 masses
-  // at 24^3x48: 1696 ms per call against 1989 ms with groups of 8 and 4);
-  // batch_kernel -2: the fastest of 1, 6, 7, 9, 12 timed on the first step
+  // batch_kernel -1: the list hop (k_bhop_pair); -2: the fastest of 1, 6, 7, 9, 12 timed on the first step
   // with this lattice and number of systems
   const double link_site = recon ? (nl / 2) * (40.0 + 28.0) : nl * 40.0;
   const int chunk = c.opt.chunk;
@@ -648,7 +835,7 @@ void BatchEngine::launch() {
     e.inflight = true;
     return;
   }
-  int variant = c.opt.batch_kernel == -1 ? (n % 8 == 0 ? 7 : 1) : std::min(c.opt.batch_kernel, N_BHOP - 1);
+  int variant = c.opt.batch_kernel == -1 ? 1 : std::min(c.opt.batch_kernel, N_BHOP - 1);
   if (c.opt.batch_kernel == -2) {
     const std::array<int, 7> key{g.L[0], g.L[1], g.L[2], g.L[3], nl, recon ? 1 : 0, n};
     auto it = g_bhop_tuned.find(key);
@@ -666,6 +853,12 @@ void BatchEngine::launch() {
            g.L[1], g.L[2], g.L[3]);
     }
   }
+  // the default hop takes the running systems from a list (k_bhop_pair); the
+  // numbered variants walk all slots
+  const bool ab = c.opt.batch_kernel == -1;
+  BList bl{};
+  for (int j = 0; j < n; j++)
+    if (e.sys[j].busy && e.h[j].flag != MIX_DONE) bl.s[bl.n++] = j;
   const int BG = kBhop[variant].bg;
   const int ngrp = (n + BG - 1) / BG;
   char hname[32];
@@ -675,18 +868,27 @@ void BatchEngine::launch() {
   for (int k = 0; k < chunk; k++) {
     {
       ProfScope s1(hname, hop_bytes);
-      launch_bhop<1>(variant, nl, recon, ngrp, nsb, e.ts, e.ps, (const unsigned char *)lk_q.a, nullptr, g, e.ng, q,
+      if (ab)
+        launch_bhop_list<1>(k > 0, nl, recon, nsb, e.ts, e.ps, (const unsigned char *)lk_q.a, nullptr, g, e.ng, q, e.dst,
+                          bl, e.part, e.count, c_long);
+      else
+        launch_bhop<1>(variant, nl, recon, ngrp, nsb, e.ts, e.ps, (const unsigned char *)lk_q.a, nullptr, g, e.ng, q,
                      e.dst, n, e.part, e.count, c_long);
       recs.push_back(s1.idx);
     }
     {
       ProfScope s2(hname, hop_bytes + (double)Vh * 16 * active);
-      launch_bhop<2>(variant, nl, recon, ngrp, nsb, e.Aps, e.ts, (const unsigned char *)lk_p.a, e.ps, g, e.ng, p,
+      if (ab)
+        launch_bhop_list<2>(true, nl, recon, nsb, e.Aps, e.ts, (const unsigned char *)lk_p.a, e.ps, g, e.ng, p, e.dst, bl,
+                          e.part, e.count, c_long);
+      else
+        launch_bhop<2>(variant, nl, recon, ngrp, nsb, e.Aps, e.ts, (const unsigned char *)lk_p.a, e.ps, g, e.ng, p,
                      e.dst, n, e.part, e.count, c_long);
       recs.push_back(s2.idx);
     }
-    k_bupdate<<<dim3(gridv, n), 256, 0, c.s>>>(e.xs, e.rs, e.ps, e.Aps, Vh, e.dst, e.part, e.count);
-    k_bp<<<dim3(gridv, n), 256, 0, c.s>>>(e.ps, e.rs, Vh, e.dst);
+    launch_k(true, k_bupdate, dim3(gridv, bl.n), 256, c.s, e.xs, e.rs, (const uint4 *)e.ps, (const uint4 *)e.Aps, Vh,
+             e.dst, bl, e.part, e.count);
+    launch_k(true, k_bp, dim3(gridv, bl.n), 256, c.s, e.ps, (const uint4 *)e.rs, Vh, (const MixState *)e.dst, bl);
     QLAUNCHN(4);
   }
   QCHECK(cudaMemcpyAsync(e.hd, e.dst, sizeof(MixState) * n, cudaMemcpyDeviceToHost, c.s));
@@ -759,7 +961,7 @@ std::vector<int> BatchEngine::collect() {
   QCHECK(cudaMemcpyAsync(e.dst, h, sizeof(MixState) * n, cudaMemcpyHostToDevice, c.s));
   for (int j : pupd) {
     if (e.tc) launch_b16_p(e.bps, e.brs, Vh, e.dst, n, j);
-    else k_bp<<<dim3(gridv, 1), 256, 0, c.s>>>(e.ps + j * Vh, e.rs + j * Vh, Vh, e.dst + j);
+    else k_bp<<<dim3(gridv, 1), 256, 0, c.s>>>(e.ps, e.rs, Vh, e.dst, BList{1, {j}});
     QLAUNCH();
   }
   return fin;
@@ -942,7 +1144,10 @@ extern "C" int QOPB_D3_sloppy_ddagd_batch(QOP_info_t *info, QOP_D3_FermionLinksA
     if (variant == N_BHOP)
       return sloppy_ddagd_batch_tc(info, reinterpret_cast<FlaT<double> *>(asqtad), n, masses, t_out, ap_out, in, eo,
                                    sums);
-    if (variant < 0) variant = n % 8 == 0 ? 7 : 1;
+    const bool ab = variant < 0;
+    if (ab) variant = 1;
+    BList bl{};
+    for (int j = 0; j < n; j++) bl.s[bl.n++] = j;
     FlaT<double> *f = reinterpret_cast<FlaT<double> *>(asqtad);
     Context &c = ctx();
     const Geom &g = c.g;
@@ -956,9 +1161,9 @@ extern "C" int QOPB_D3_sloppy_ddagd_batch(QOP_info_t *info, QOP_D3_FermionLinksA
     ts = dalloc<uint4>(n * Vh);
     as = dalloc<uint4>(n * Vh);
     dst = dalloc<MixState>(n);
-    part = dalloc<double>((size_t)ngrp * BG * nsb);
-    count = dalloc<unsigned>(ngrp);
-    dzero(count, sizeof(unsigned) * ngrp);
+    part = dalloc<double>((size_t)(n + BATCH_MAX) * nsb);   // groups x systems per group <= n + 15
+    count = dalloc<unsigned>(BATCH_MAX);
+    dzero(count, sizeof(unsigned) * BATCH_MAX);
     std::vector<MixState> h(n);
     for (int j = 0; j < n; j++) {
       h[j] = MixState{};
@@ -979,12 +1184,20 @@ extern "C" int QOPB_D3_sloppy_ddagd_batch(QOP_info_t *info, QOP_D3_FermionLinksA
     const double tb = (double)Vh * ((recon ? (sl->nl / 2) * (40.0 + 28.0) : sl->nl * 40.0) + 2.0 * 16 * n);
     {
       ProfScope s1("check_bhop_q16", tb);
+      if (ab)
+        launch_bhop_list<1>(false, sl->nl, recon, nsb, ts, ps, (const unsigned char *)lk_q.a, nullptr, g, ng, q, dst, bl,
+                          part, count, c_long);
+      else
       launch_bhop<1>(variant, sl->nl, recon, ngrp, nsb, ts, ps, (const unsigned char *)lk_q.a, nullptr, g, ng, q, dst,
                      n, part, count, c_long);
       QLAUNCH();
     }
     {
       ProfScope s2("check_bhop_q16", tb + (double)Vh * 16 * n);
+      if (ab)
+        launch_bhop_list<2>(false, sl->nl, recon, nsb, as, ts, (const unsigned char *)lk_p.a, ps, g, ng, p, dst, bl, part,
+                          count, c_long);
+      else
       launch_bhop<2>(variant, sl->nl, recon, ngrp, nsb, as, ts, (const unsigned char *)lk_p.a, ps, g, ng, p, dst, n,
                      part, count, c_long);
       QLAUNCH();
