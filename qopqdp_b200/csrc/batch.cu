@@ -481,7 +481,8 @@ k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState 
   SpQ16::store(p + o, i, Vh, pv);
 }
 
-// batched hop variants (option batch_kernel): systems per thread, the
+// numbered batched hop variants (option batch_kernel; the default is the list
+// hop above): systems per thread, the
 // register cap (resident blocks per SM) and the slot unrolling.  At 32^4
 // with 16 systems a hop takes 531 us with variant 7 (8 systems per thread,
 // 3 blocks per SM, slot loop unrolled by 2), 557-580 us with
@@ -492,8 +493,7 @@ k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState 
 // instruction- and latency-bound, not HBM-bound.  12-15 use the packed pair
 // form of the one-system hop (q16_pk_mul): 550 us with 4 systems per thread
 // (12, against 577 for 1), but 625 / 810 us with 8 (13 / 14: two
-// accumulators per row and system exceed the register budget), so 7 stays
-// the choice for 16 systems; at 24^3x48 with 12 systems 12 and 1 tie
+// accumulators per row and system exceed the register budget); at 24^3x48 with 12 systems 12 and 1 tie
 // (114.0 / 113.8 us).
 struct BhopShape { int bg, minb; };
 static const BhopShape kBhop[] = {{4, 1}, {4, 5}, {2, 8}, {2, 1}, {8, 1}, {4, 6}, {4, 5}, {8, 3}, {8, 2},
