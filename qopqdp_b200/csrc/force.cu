@@ -90,7 +90,8 @@ __device__ __forceinline__ void adj_link_row(const Geom &g, const StSite &s, con
 
 // The derivative for one direction mu from its chains (staple.cuh): groups
 // 0-2 add the adjoint of U_n, n != mu, to D_n; group 3 adds the adjoint of
-// the starting link, c1 M + w sum_n staple(Y_n; n), to D_mu
+// the starting link, c1 M + w sum_n staple(Y_n; n), to D_mu; NG groups from
+// the g0-th on
 struct SweepArgs {
   AdjPairs pr[3];
   int np;
@@ -98,9 +99,10 @@ struct SweepArgs {
   double2 *D[4];
   double c1, w;
 };
-__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_sweep(const __grid_constant__ SweepArgs a, const __grid_constant__ StU U, int mu, Geom g) {
+template <int NG>
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_sweep(const __grid_constant__ SweepArgs a, const __grid_constant__ StU U, int mu, int g0, Geom g) {
   int grp, p, i;
-  if (!st_block(g, 4, grp, p, i)) return;
+  if (!st_block<NG>(g, g0, grp, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y;
   const i64 Vh = g.Vh;
@@ -120,15 +122,16 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_sweep(const __grid_co
   }
 }
 
-// adjoint of long(x) = c U(x) U(x+mu) U(x+2mu), the directions as groups:
+// adjoint of long(x) = c U(x) U(x+mu) U(x+2mu), NG directions from mu0 on as groups:
 // D(z) += c [N(z) (U(z+mu) U(z+2mu))^+ + U(z-mu)^+ N(z-mu) U(z+mu)^+ + (U(z-2mu) U(z-mu))^+ N(z-2mu)]
 struct NaikAdjArgs {
   double2 *D[4];
   const double2 *N[4];
 };
-__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_adj_naik(const __grid_constant__ NaikAdjArgs a, const __grid_constant__ StU Us, double c, Geom g) {
+template <int NG>
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_adj_naik(const __grid_constant__ NaikAdjArgs a, const __grid_constant__ StU Us, double c, int mu0, Geom g) {
   int mu, p, i;
-  if (!st_block(g, 4, mu, p, i)) return;
+  if (!st_block<NG>(g, mu0, mu, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y, q = 1 - p;
   const i64 Vh = g.Vh;
@@ -215,17 +218,18 @@ __global__ void k_field_axpby(double2 *d, double a, const double2 *s, double b, 
 
 // midF_mu(x) = sgn(x) sum_i eps_i x_i(x) x_i(x+mu)^+ (midN: x+3mu) with
 // sgn = even_sign on even and -even_sign on odd sites (asqtad: -1, HISQ: +1);
-// vectors are [parity][colour][site]
+// vectors are [parity][colour][site]; directions mu0 .. mu1 - 1, the fields
+// from mu0 on; midF or midN may be null
 template <typename T>
 __global__ void k_force_mid(double2 *midF, double2 *midN, const c2<T> *const *xs, const double *eps, int nsrc,
-                            double even_sign, Geom g) {
+                            double even_sign, int mu0, int mu1, Geom g) {
   const i64 s = blockIdx.x * (i64)blockDim.x + threadIdx.x;
   if (s >= 2 * g.Vh) return;
   int p, i, x[4];
   site_of(g, s, p, i, x);
   const double sgn = p ? -even_sign : even_sign;
   const i64 Vh = g.Vh;
-  for (int mu = 0; mu < 4; mu++) {
+  for (int mu = mu0; mu < mu1; mu++) {
     for (int k = 0; k < 2; k++) {
       double2 *out = k == 0 ? midF : midN;
       if (!out) continue;
@@ -252,7 +256,7 @@ __global__ void k_force_mid(double2 *midF, double2 *midN, const c2<T> *const *xs
             m.e[3 * r + c].y += w * (a[r].y * b[c].x - a[r].x * b[c].y);
           }
       }
-      st3(out + (i64)mu * 18 * Vh + (i64)p * 9 * Vh + i, Vh, m);
+      st3(out + (i64)(mu - mu0) * 18 * Vh + (i64)p * 9 * Vh + i, Vh, m);
     }
   }
 }
@@ -380,11 +384,8 @@ __global__ void k_reunit_adj(double2 *GV, const double2 *V, const double2 *GW, i
 // path took 64 launches and about 300; 24^3 x 48, HISQ, 8 sources: the call
 // takes 27.0 ms against 62.1 (8^4 asqtad, 2 sources: 0.17 against 1.68).
 // The sweep kernel runs the FP64 pipe at 43 % and L1 at 51 % of their rates;
-// the latency of L2 reads at 15 warps per SM is the rest.  lepage_rep adds the reference's Lepage term
-// of the form U H (k_lep_h), for a derivative that feeds something other
-// than the force projection.  work: SWEEP_FIELDS fields [2][9][Vh].
-// Returns sweep_terms.
-constexpr int SWEEP_FIELDS = 12;
+// the latency of L2 reads at 15 warps per SM is the rest.
+constexpr int SWEEP_FIELDS = 12, SWEEP_LEAN = 7;   // work fields [2][9][Vh]
 // staple applications and field sums of the sweep walked path by path: the
 // unit of the flops that the force calls report
 int sweep_terms(const double c[6], bool naik, bool lepage_rep) {
@@ -392,67 +393,114 @@ int sweep_terms(const double c[6], bool naik, bool lepage_rep) {
   const int per_nu = 4 + (c[4] != 0 ? 2 : 0) + (have5 ? 2 * (4 + (c[3] != 0 ? 2 : 0)) : 0);
   return 4 * (1 + (have3 ? 3 * per_nu : 0)) + (naik && c[5] != 0 ? 4 : 0) + (lepage_rep && c[4] != 0 ? 8 : 0);
 }
+
+// The contributions of direction mu, M = midF_mu.  nx = 3: work holds
+// SWEEP_FIELDS fields; nx = 1: SWEEP_LEAN (S_n, A_n and one field that takes
+// I_n and then X_n of one n after the other), with twelve more launches.
+void sweep_dir(const StU &Us, const double c[6], int mu, const double2 *M, double2 *D, double2 *work, int nx) {
+  Context &cx = ctx();
+  const Geom &g = cx.g;
+  const cudaStream_t st = cx.s;
+  const i64 F1 = 18 * g.Vh;
+  const double c1 = c[0] - 6 * c[4], c3 = c[1], c5 = c[2], c7 = c[3], cL = c[4];
+  const bool have5 = c5 != 0 || c7 != 0 || cL != 0, have3 = c3 != 0 || have5;
+  if (!have3) {
+    k_field_axpby<<<grid_for(F1, 256), 256, 0, st>>>(D + mu * F1, 1.0, M, c1, F1);
+    QLAUNCH();
+    return;
+  }
+  const double2 *const Umu = Us.d[mu];
+  SweepArgs a{};
+  for (int d = 0; d < 4; d++) a.D[d] = D + d * F1;
+  a.M = M;
+  a.c1 = c1;
+  if (!have5) {   // three-link staples only: X_n = c3 M
+    a.np = 1;
+    a.w = c3;
+    for (int j = 0; j < 3; j++) {
+      a.pr[j] = AdjPairs{{M}, {Umu}, {c3}};
+      a.Y[j] = M;
+    }
+    k_sweep<4><<<st_grid(g, 4), st_threads(), 0, st>>>(a, Us, mu, 0, g);
+    QLAUNCH();
+    return;
+  }
+  const StCoef co{cL, c5, c7};
+  a.w = 1.0;
+  StChain<2> ch;
+  ch.in[0] = Umu;
+  ch.in[1] = M;
+  ch.c3[0] = 0;
+  ch.c3[1] = c3;
+  for (int f = 0; f < 2; f++)
+    for (int j = 0; j < 3; j++) {
+      ch.S[f][j] = work + ((nx == 3 ? 6 : 3) * f + j) * F1;
+      ch.X[f][j] = work + (nx == 3 ? 6 * f + 3 + j : 6) * F1;
+    }
+  k_chain_s<2><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, Us, mu, g);
+  QLAUNCH();
+  // r, s: the other two of the three directions
+  auto r_of = [](int j) { return j == 0 ? 1 : 0; };
+  auto s_of = [](int j) { return j == 2 ? 1 : 2; };
+  if (nx == 3) {
+    k_chain_x<2, 3><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, Us, co, mu, 0, g);
+    a.np = c7 != 0 ? 4 : 2;
+    for (int j = 0; j < 3; j++) {
+      a.pr[j] = AdjPairs{{M, ch.X[1][j], ch.S[1][s_of(j)], ch.S[1][r_of(j)]},
+                         {ch.X[0][j], Umu, ch.S[0][r_of(j)], ch.S[0][s_of(j)]},
+                         {1.0, 1.0, c7, c7}};
+      a.Y[j] = ch.X[1][j];
+    }
+    k_sweep<4><<<st_grid(g, 4), st_threads(), 0, st>>>(a, Us, mu, 0, g);
+    QLAUNCHN(2);
+    return;
+  }
+  for (int j = 0; j < 3; j++) {
+    double2 *X = ch.X[0][j];
+    for (int f = 0; f < 2; f++) {   // X = I_n, then X_n
+      StChain<1> one;
+      one.in[0] = ch.in[f];
+      one.c3[0] = ch.c3[f];
+      for (int k = 0; k < 3; k++) {
+        one.S[0][k] = ch.S[f][k];
+        one.X[0][k] = X;
+      }
+      k_chain_x<1, 1><<<st_grid(g, 1), st_threads(), 0, st>>>(one, Us, co, mu, j, g);
+      if (f == 0) {
+        a.np = c7 != 0 ? 3 : 1;
+        a.pr[j] = AdjPairs{{M, ch.S[1][s_of(j)], ch.S[1][r_of(j)]}, {X, ch.S[0][r_of(j)], ch.S[0][s_of(j)]}, {1.0, c7, c7}};
+      } else {
+        a.np = 1;
+        a.pr[j] = AdjPairs{{X}, {Umu}, {1.0}};
+        for (int k = 0; k < 3; k++) a.Y[k] = k == j ? X : nullptr;
+        a.c1 = j == 0 ? c1 : 0.0;
+        k_sweep<1><<<st_grid(g, 1), st_threads(), 0, st>>>(a, Us, mu, 3, g);
+        QLAUNCH();
+      }
+      k_sweep<1><<<st_grid(g, 1), st_threads(), 0, st>>>(a, Us, mu, j, g);
+      QLAUNCHN(2);
+    }
+  }
+}
+
+// lepage_rep adds the reference's Lepage term of the form U H (k_lep_h), for a
+// derivative that feeds something other than the force projection.  work:
+// SWEEP_FIELDS fields.  Returns sweep_terms.
 int smear_adjoint(const double2 *U, const double c[6], const double2 *mid, const double2 *midN, double2 *D,
                   double2 *work, bool lepage_rep = false) {
   Context &cx = ctx();
   const Geom &g = cx.g;
   const i64 F1 = 18 * g.Vh;
-  const int grid2 = grid_for(2 * g.Vh, 128), gridF = grid_for(F1, 256);
-  const double c1 = c[0] - 6 * c[4], c3 = c[1], c5 = c[2], c7 = c[3], cL = c[4];
-  const bool have5 = c5 != 0 || c7 != 0 || cL != 0, have3 = c3 != 0 || have5;
+  const int grid2 = grid_for(2 * g.Vh, 128);
+  const double cL = c[4];
   auto Uf = [&](int d) { return U + d * F1; };
   auto Df = [&](int d) { return D + d * F1; };
   const StU Us{{Uf(0), Uf(1), Uf(2), Uf(3)}};
-  int nk = 0;
-  for (int mu = 0; mu < 4; mu++) {
-    const double2 *M = mid + mu * F1;
-    if (!have3) {
-      k_field_axpby<<<gridF, 256, 0, cx.s>>>(Df(mu), 1.0, M, c1, F1);
-      nk++;
-      continue;
-    }
-    SweepArgs a{};
-    for (int d = 0; d < 4; d++) a.D[d] = Df(d);
-    a.M = M;
-    a.c1 = c1;
-    if (have5) {
-      StChain<2> ch;
-      ch.in[0] = Uf(mu);
-      ch.in[1] = M;
-      ch.c3[0] = 0;
-      ch.c3[1] = c3;
-      for (int f = 0; f < 2; f++)
-        for (int j = 0; j < 3; j++) {
-          ch.S[f][j] = work + (6 * f + j) * F1;
-          ch.X[f][j] = work + (6 * f + 3 + j) * F1;
-        }
-      k_chain_s<2><<<st_grid(g, 3), st_threads(), 0, cx.s>>>(ch, Us, mu, g);
-      k_chain_x<2><<<st_grid(g, 3), st_threads(), 0, cx.s>>>(ch, Us, StCoef{cL, c5, c7}, mu, g);
-      nk += 2;
-      a.np = c7 != 0 ? 4 : 2;
-      a.w = 1.0;
-      for (int j = 0; j < 3; j++) {
-        const int j1 = j == 0 ? 1 : 0, j2 = j == 2 ? 1 : 2;
-        a.pr[j] = AdjPairs{{M, ch.X[1][j], ch.S[1][j2], ch.S[1][j1]},
-                           {ch.X[0][j], Uf(mu), ch.S[0][j1], ch.S[0][j2]},
-                           {1.0, 1.0, c7, c7}};
-        a.Y[j] = ch.X[1][j];
-      }
-    } else {   // three-link staples only: X_n = c3 M
-      a.np = 1;
-      a.w = c3;
-      for (int j = 0; j < 3; j++) {
-        a.pr[j] = AdjPairs{{M}, {Uf(mu)}, {c3}};
-        a.Y[j] = M;
-      }
-    }
-    k_sweep<<<st_grid(g, 4), st_threads(), 0, cx.s>>>(a, Us, mu, g);
-    nk++;
-  }
+  for (int mu = 0; mu < 4; mu++) sweep_dir(Us, c, mu, mid + mu * F1, D, work, 3);
   if (midN && c[5] != 0) {
-    k_adj_naik<<<st_grid(g, 4), st_threads(), 0, cx.s>>>(
-        NaikAdjArgs{{Df(0), Df(1), Df(2), Df(3)}, {midN, midN + F1, midN + 2 * F1, midN + 3 * F1}}, Us, c[5], g);
-    nk++;
+    k_adj_naik<4><<<st_grid(g, 4), st_threads(), 0, cx.s>>>(
+        NaikAdjArgs{{Df(0), Df(1), Df(2), Df(3)}, {midN, midN + F1, midN + 2 * F1, midN + 3 * F1}}, Us, c[5], 0, g);
+    QLAUNCH();
   }
   if (lepage_rep && cL != 0) {
     double2 *H[4] = {work, work + F1, work + 2 * F1, work + 3 * F1};   // free once the sweep is done
@@ -463,30 +511,61 @@ int smear_adjoint(const double2 *U, const double c[6], const double2 *mid, const
         if (nu != mu) o[k++] = H[nu];
       k_lep_fix<<<grid2, 128, 0, cx.s>>>(Df(mu), Uf(mu), o[0], o[1], o[2], mu, cL, g);
     }
-    nk += 8;
+    QLAUNCHN(8);
   }
-  QLAUNCHN(nk);
   return sweep_terms(c, midN != nullptr, lepage_rep);
 }
 
-// outer products of sources [first, first + n) into mid (and midN)
-template <typename T>
-void force_mids(double2 *mid, double2 *midN, VecT<T> *const *x, const double *w, int n, double even_sign) {
-  Context &cx = ctx();
-  std::vector<const c2<T> *> hx(n);
-  for (int k = 0; k < n; k++) hx[k] = x[k]->d;
-  const c2<T> **dx = dalloc<const c2<T> *>(n);
-  double *dw = dalloc<double>(n);
-  QCHECK(cudaMemcpyAsync(dx, hx.data(), sizeof(void *) * n, cudaMemcpyHostToDevice, cx.s));
-  QCHECK(cudaMemcpyAsync(dw, w, sizeof(double) * n, cudaMemcpyHostToDevice, cx.s));
-  k_force_mid<T><<<grid_for(2 * cx.g.Vh, 128), 128, 0, cx.s>>>(mid, midN, dx, dw, n, even_sign, cx.g);
-  QLAUNCH();
-  dfree(dx);
-  dfree(dw);
-}
+// a device allocation freed at the end of its scope
+template <typename E> struct Buf {
+  E *p = nullptr;
+  Buf() = default;
+  explicit Buf(i64 n) : p(dalloc<E>(n)) {}
+  Buf(const Buf &) = delete;
+  Buf &operator=(const Buf &) = delete;
+  ~Buf() { dfree((void *)p); }
+  operator E *() const { return p; }
+};
+
+// the sources of a force call on the device
+template <typename T> struct ForceSources {
+  Buf<const c2<T> *> x;
+  Buf<double> w;
+  int n;
+  ForceSources(VecT<T> *const *v, const double *weight, int n_) : x(n_), w(n_), n(n_) {
+    std::vector<const c2<T> *> hx(n);
+    for (int k = 0; k < n; k++) hx[k] = v[k]->d;
+    QCHECK(cudaMemcpyAsync(x, hx.data(), sizeof(void *) * n, cudaMemcpyHostToDevice, ctx().s));
+    QCHECK(cudaMemcpyAsync(w, weight, sizeof(double) * n, cudaMemcpyHostToDevice, ctx().s));
+  }
+  // their outer products along the directions mu0 .. mu1 - 1
+  void mids(double2 *midF, double2 *midN, double even_sign, int mu0 = 0, int mu1 = 4) const {
+    const Geom &g = ctx().g;
+    k_force_mid<T><<<grid_for(2 * g.Vh, 128), 128, 0, ctx().s>>>(midF, midN, x, w, n, even_sign, mu0, mu1, g);
+    QLAUNCH();
+  }
+};
+
+// a gauge field in FP64: the field itself, or a copy freed at the end of the scope
+struct Gauge64 {
+  double2 *p;
+  bool own = false;
+  template <typename T> explicit Gauge64(GaugeT<T> *G) { p = gauge_fp64(G, own); }
+  Gauge64(const Gauge64 &) = delete;
+  Gauge64 &operator=(const Gauge64 &) = delete;
+  ~Gauge64() {
+    if (own) dfree(p);
+  }
+  operator double2 *() const { return p; }
+};
 
 }  // namespace
 
+// Scratch: D and, where they fit, every outer product (4 fields, 8 with the
+// Naik term) and the sweep's 12; otherwise one direction's outer product at a
+// time and SWEEP_LEAN, 12 fields in all, so that every lattice on which a walk
+// over single paths fits (4 work fields: 12, or 16 with the Naik term) is
+// still taken.
 template <typename T>
 void asqtad_force(QOP_info_t *info, GaugeT<T> *G, GaugeT<T> *F, const QOP_asqtad_coeffs_t *cf, const double *eps,
                   VecT<T> *const *x, int nsrc) {
@@ -494,15 +573,33 @@ void asqtad_force(QOP_info_t *info, GaugeT<T> *G, GaugeT<T> *F, const QOP_asqtad
   const Geom &g = c.g;
   const double t0 = wtime();
   const i64 Vh = g.Vh, F1 = 18 * Vh, F4 = 72 * Vh;
-  bool own = false;
-  double2 *U = gauge_fp64(G, own);
+  const Gauge64 U(G);
   const bool naik = cf->naik != 0;
-  double2 *mid = dalloc<double2>(naik ? 2 * F4 : F4), *D = dalloc<double2>(F4);
-  dzero(D, sizeof(double2) * F4);
-  double2 *w = dalloc<double2>(SWEEP_FIELDS * F1);
-  force_mids<T>(mid, naik ? mid + F4 : nullptr, x, eps, nsrc, -1.0);   // scale -1 (fnmat_p.c:497)
   const double co[6] = {cf->one_link, cf->three_staple, cf->five_staple, cf->seven_staple, cf->lepage, cf->naik};
-  const int nk = smear_adjoint(U, co, mid, naik ? mid + F4 : nullptr, D, w);
+  const ForceSources<T> src(x, eps, nsrc);
+  Buf<double2> D(F4), w;
+  dzero(D, sizeof(double2) * F4);
+  const i64 nmid = naik ? 8 : 4;
+  int nx = 3;
+  w.p = st_workspace(F1, (int)nmid + SWEEP_FIELDS, 1 + SWEEP_LEAN, nx);
+  if (nx == 3) {
+    double2 *mid = w, *midN = naik ? mid + F4 : nullptr;
+    src.mids(mid, midN, -1.0);   // scale -1 (fnmat_p.c:497)
+    smear_adjoint(U, co, mid, midN, D, w + nmid * F1);
+  } else {
+    const StU Us{{U, U + F1, U + 2 * F1, U + 3 * F1}};
+    for (int mu = 0; mu < 4; mu++) {
+      src.mids(w, nullptr, -1.0, mu, mu + 1);
+      sweep_dir(Us, co, mu, w, D, w + F1, nx);
+      if (!naik) continue;
+      src.mids(nullptr, w, -1.0, mu, mu + 1);
+      NaikAdjArgs a{};
+      a.D[mu] = D + mu * F1;
+      a.N[mu] = w;
+      k_adj_naik<1><<<st_grid(g, 1), st_threads(), 0, c.s>>>(a, Us, co[5], mu, g);
+      QLAUNCH();
+    }
+  }
   // the reference's algorithm choice (lib/asqtad_force_p.c:22): FNMAT adds
   // -2 TA(U D^+); ASVEC (fewer sources than fnmat_src_min) stores
   // TA(force + C) with TA(C) = -TA(U D^+), half the FNMAT term
@@ -514,16 +611,17 @@ void asqtad_force(QOP_info_t *info, GaugeT<T> *G, GaugeT<T> *F, const QOP_asqtad
   k_force_ta<T><<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(F->d, U, D, asvec ? -1.0 : -2.0, g);
   QLAUNCH();
   sync();
-  dfree(mid); dfree(D); dfree(w);
-  if (own) dfree(U);
   if (info) {
     info->final_sec = wtime() - t0;
     // outer products, adjoint staples (~4 matrix products each) and projection
-    info->final_flop = (double)g.V * (4.0 * (naik ? 2 : 1) * 72 * nsrc + nk * 216.0 + 4 * 264);
+    info->final_flop = (double)g.V * (4.0 * (naik ? 2 : 1) * 72 * nsrc + sweep_terms(co, naik, false) * 216.0 + 4 * 264);
     info->status = QOP_SUCCESS;
   }
 }
 
+// Scratch: 24 fields.  The W level holds the outer products (8), the adjoint
+// of W (4) and the sweep's 12; the U level sweeps in the first 12, with the
+// adjoint of V and the derivative in the other 12.
 template <typename T>
 void hisq_force(QOP_info_t *info, HisqT<T> *h, GaugeT<T> *F, const QOP_hisq_coeffs_t *cf, const double *res,
                 VecT<T> *const *x, const int *n_orders) {
@@ -534,13 +632,11 @@ void hisq_force(QOP_info_t *info, HisqT<T> *h, GaugeT<T> *F, const QOP_hisq_coef
     fail(QOP_FAIL, "hisq_force: the HISQ links carry no auxiliary U/V/W fields "
                    "(create them with QOP_hisq_links_set_opts want_aux = 1)");
   const i64 Vh = g.Vh, F1 = 18 * Vh, F4 = 72 * Vh;
-  bool oU = false, oV = false, oW = false;
-  double2 *U = gauge_fp64(h->U, oU), *V = gauge_fp64(h->V, oV), *W = gauge_fp64(h->W, oW);
-  double2 *mid = dalloc<double2>(2 * F4), *GW = dalloc<double2>(F4), *T1 = dalloc<double2>(F4);
-  double2 *D = dalloc<double2>(F4);
+  static_assert(SWEEP_FIELDS == 12, "the two halves of the scratch trade places");
+  const Gauge64 U(h->U), V(h->V), W(h->W);
+  Buf<double2> mid(SWEEP_FIELDS * F1), w(SWEEP_FIELDS * F1);
+  double2 *GW = mid + 2 * F4, *GV = w, *D = w + F4;
   dzero(GW, sizeof(double2) * F4);
-  dzero(D, sizeof(double2) * F4);
-  double2 *w = dalloc<double2>(SWEEP_FIELDS * F1);
   int nterms = 0;
   for (int k = 0; k < cf->n_naiks; k++) nterms += n_orders[k];
   const double ca[6] = {cf->asqtad_one_link, cf->asqtad_three_staple, cf->asqtad_five_staple,
@@ -549,28 +645,27 @@ void hisq_force(QOP_info_t *info, HisqT<T> *h, GaugeT<T> *F, const QOP_hisq_coef
   int nk = 0, shift = 0;
   for (int k = 0; k < cf->n_naiks; k++) {
     // group 0 takes every source with the asqtad coefficients, group k >= 1
-    // its own sources with the difference coefficients (fnmat2_p.c:52-113)
+    // its own sources with the difference coefficients (fnmat2_p.c:52-113),
+    // its eps_naik folded into the weights (the derivative is linear in them)
     const int first = k == 0 ? 0 : shift, count = k == 0 ? nterms : n_orders[k];
     shift += n_orders[k];
     if (count == 0) continue;
-    force_mids<T>(mid, mid + F4, x + first, res + first, count, 1.0);
-    dzero(T1, sizeof(double2) * F4);
-    nk += smear_adjoint(W, k == 0 ? ca : cd, mid, mid + F4, T1, w, true);
-    k_field_axpby<<<grid_for(F4, 256), 256, 0, c.s>>>(GW, 1.0, T1, k == 0 ? 1.0 : cf->eps_naik[k], F4);
-    QLAUNCH();
+    std::vector<double> wt(res + first, res + first + count);
+    if (k > 0)
+      for (double &v : wt) v *= cf->eps_naik[k];
+    const ForceSources<T> src(x + first, wt.data(), count);
+    src.mids(mid, mid + F4, 1.0);
+    nk += smear_adjoint(W, k == 0 ? ca : cd, mid, mid + F4, GW, w, true);
   }
-  k_reunit_adj<<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(T1, V, GW, 8 * Vh, c.opt.hisq_force_filter);   // T1 = GV
+  k_reunit_adj<<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(GV, V, GW, 8 * Vh, c.opt.hisq_force_filter);
   QLAUNCH();
   const double c7[6] = {cf->fat7_one_link, cf->fat7_three_staple, cf->fat7_five_staple, cf->fat7_seven_staple,
                         c.opt.use_fat7_lepage ? cf->fat7_lepage : 0.0, 0.0};
-  nk += smear_adjoint(U, c7, T1, nullptr, D, w);
+  dzero(D, sizeof(double2) * F4);
+  nk += smear_adjoint(U, c7, GV, nullptr, D, mid);
   k_force_ta<T><<<grid_for(8 * Vh, 128), 128, 0, c.s>>>(F->d, U, D, 2.0, g);   // deriv = 2 D
   QLAUNCH();
   sync();
-  dfree(mid); dfree(GW); dfree(T1); dfree(D); dfree(w);
-  if (oU) dfree(U);
-  if (oV) dfree(V);
-  if (oW) dfree(W);
   if (info) {
     info->final_sec = wtime() - t0;
     info->final_flop = (double)g.V * (8.0 * 72 * nterms + nk * 216.0 + 4 * 1500 + 4 * 264);

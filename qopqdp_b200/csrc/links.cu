@@ -16,7 +16,8 @@ namespace qopb {
 
 
 // ---------------------------------------------------------------- staples
-// fl = c1 in + w sum_n staple(Y_n; n)  (staple.cuh; w 0: no staples)
+// fl = c1 in + w sum_n staple(Y_n; n)  (staple.cuh; `in` may be fl: a thread
+// reads the elements that it writes)
 struct FatArgs {
   const double2 *in, *Y[3];
   double2 *fl;
@@ -24,7 +25,7 @@ struct FatArgs {
 };
 __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_fat(const __grid_constant__ FatArgs f, const __grid_constant__ StU U, int mu, Geom g) {
   int grp, p, i;
-  if (!st_block(g, 1, grp, p, i)) return;
+  if (!st_block<1>(g, 0, grp, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y;
   const i64 Vh = g.Vh;
@@ -33,6 +34,16 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_fat(const __grid_cons
   double2 *o = st_at(f.fl, Vh, p, s.lex);
 #pragma unroll
   for (int c = 0; c < 3; c++) o[(3 * r + c) * Vh] = a[0][c];
+}
+
+double2 *st_workspace(i64 F, int most, int least, int &per) {
+  try {
+    return dalloc<double2>(most * F);
+  } catch (const Fail &e) {
+    if (e.status != QOP_MEM_ERROR) throw;
+  }
+  per = 1;
+  return dalloc<double2>(least * F);
 }
 
 __global__ void k_scale_field(double2 *d, const double2 *s, double c, i64 n) {
@@ -48,7 +59,7 @@ struct NaikArgs {
 };
 __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_naik(const __grid_constant__ NaikArgs n, const __grid_constant__ StU U, double naik, Geom g) {
   int mu, p, i;
-  if (!st_block(g, 4, mu, p, i)) return;
+  if (!st_block<4>(g, 0, mu, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y;
   const i64 Vh = g.Vh;
@@ -67,6 +78,10 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_naik(const __grid_con
 // 12 staples and about 25 field passes where 18 staples took about 95.  The
 // latency of the L2 reads bounds them (24^3 x 48, HISQ: the whole call 9.4 ms
 // against 22.4 with one launch per staple; 12^4: 0.44 against 1.35 ms).
+// Work fields: three S_n and three X_n.  Where six do not fit, one X_n at a
+// time is formed and added (four fields): with the finished links (eight
+// slots of FP32 are four such fields) no lattice needs more than the largest
+// sum of its outputs.
 static double make_imp_links(const QOP_asqtad_coeffs_t *cf, const double2 *gf, const double2 *gfLong, double2 *fl,
                              double2 *ll) {
   const Geom &g = ctx().g;
@@ -77,7 +92,8 @@ static double make_imp_links(const QOP_asqtad_coeffs_t *cf, const double2 *gf, c
   const bool have5 = c5 != 0 || c7 != 0 || cL != 0;
   const bool have3 = c3 != 0 || have5;
   const StU U{{gf, gf + F, gf + 2 * F, gf + 3 * F}};
-  double2 *work = have5 ? dalloc<double2>(6 * F) : nullptr;   // S_n and X_n of one direction
+  int nx = 3;   // X_n fields
+  double2 *work = have5 ? st_workspace(F, 6, 4, nx) : nullptr;
   for (int dir = 0; dir < 4; dir++) {
     const double2 *in = gf + dir * F;
     if (!have3) {
@@ -92,12 +108,24 @@ static double make_imp_links(const QOP_asqtad_coeffs_t *cf, const double2 *gf, c
       ch.c3[0] = c3;
       for (int j = 0; j < 3; j++) {
         ch.S[0][j] = work + j * F;
-        fa.Y[j] = ch.X[0][j] = work + (3 + j) * F;
+        fa.Y[j] = ch.X[0][j] = work + (3 + j % nx) * F;
       }
       fa.w = 1.0;
       k_chain_s<1><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, U, dir, g);
-      k_chain_x<1><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, U, StCoef{cL, c5, c7}, dir, g);
-      QLAUNCHN(2);
+      QLAUNCH();
+      if (nx == 1) {
+        for (int j = 0; j < 3; j++) {
+          const FatArgs one{j ? fl + dir * F : in, {j == 0 ? work + 3 * F : nullptr, j == 1 ? work + 3 * F : nullptr,
+                                                    j == 2 ? work + 3 * F : nullptr},
+                            fl + dir * F, j ? 1.0 : c1, 1.0};
+          k_chain_x<1, 1><<<st_grid(g, 1), st_threads(), 0, st>>>(ch, U, StCoef{cL, c5, c7}, dir, j, g);
+          k_fat<<<st_grid(g, 1), st_threads(), 0, st>>>(one, U, dir, g);
+          QLAUNCHN(2);
+        }
+        continue;
+      }
+      k_chain_x<1, 3><<<st_grid(g, 3), st_threads(), 0, st>>>(ch, U, StCoef{cL, c5, c7}, dir, 0, g);
+      QLAUNCH();
     }
     k_fat<<<st_grid(g, 1), st_threads(), 0, st>>>(fa, U, dir, g);
     QLAUNCH();

@@ -9,11 +9,11 @@
 // takes 12 staples per direction (18 when every path is walked by itself),
 // and the adjoint of a staple with respect to `in` is the same staple.
 //
-// One thread owns one row of one site's result (block: 64 sites x 3 rows):
+// One thread owns one row of one site's result (block: 32 sites x 3 rows):
 // row r of a product chain needs one row of the first factor and streams the
-// others, so a thread holds about 80-110 registers where a thread that owns
-// the whole 3x3 result holds 140-196, and three times as many warps cover
-// the latency of the loads.  The rows of a site re-read the other factors
+// others, so a thread fits in 128 registers (the cap of 5 resident blocks)
+// where a thread that owns the whole 3x3 result holds 140-196, and three times
+// as many threads cover the latency of the loads.  The rows of a site re-read the other factors
 // from L1.  The groups (directions n) of a site block are adjacent in the
 // grid, group fastest, then the parity, so the fields that the groups share
 // come from HBM once.
@@ -145,12 +145,14 @@ __device__ __forceinline__ void st_staple(const Geom &g, const StSite &s, const 
 // the j-th direction (j = 0, 1, 2) other than mu
 __host__ __device__ constexpr int st_dir(int mu, int j) { return j < mu ? j : j + 1; }
 
-// block -> (group, parity, site); false outside the lattice
-__device__ __forceinline__ bool st_block(const Geom &g, int ngrp, int &grp, int &p, int &i) {
+// block -> (group, parity, site); false outside the lattice.  NG groups from
+// g0 on
+template <int NG>
+__device__ __forceinline__ bool st_block(const Geom &g, int g0, int &grp, int &p, int &i) {
   const int b = blockIdx.x;
-  grp = b % ngrp;
-  p = (b / ngrp) & 1;
-  i = (b / ngrp >> 1) * ST_SITES + threadIdx.x;
+  grp = g0 + b % NG;
+  p = (b / NG) & 1;
+  i = (b / NG >> 1) * ST_SITES + threadIdx.x;
   return i < g.Vh;
 }
 inline unsigned st_grid(const Geom &g, int ngrp) {
@@ -172,11 +174,15 @@ struct StU {
   const double2 *d[4];
 };
 
+// work fields of F elements: `most` of them, or where that allocation fails
+// `least` and per = 1 (one X_n at a time; links.cu)
+double2 *st_workspace(i64 F, int most, int least, int &per);
+
 // S_n = staple(in; mu, n)
 template <int NF>
 __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_chain_s(const __grid_constant__ StChain<NF> ch, const __grid_constant__ StU U, int mu, Geom g) {
   int grp, p, i;
-  if (!st_block(g, 3, grp, p, i)) return;
+  if (!st_block<3>(g, 0, grp, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y, nu = st_dir(mu, grp);
   const i64 Vh = g.Vh;
@@ -191,10 +197,11 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_chain_s(const __grid_
 }
 
 // X_n = c3 in + cL S_n + c5 (S_r + S_s) + c7 (staple(S_r; s) + staple(S_s; r))
-template <int NF>
-__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_chain_x(const __grid_constant__ StChain<NF> ch, const __grid_constant__ StU U, StCoef co, int mu, Geom g) {
+// for the NG directions n from the g0-th on
+template <int NF, int NG>
+__global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_chain_x(const __grid_constant__ StChain<NF> ch, const __grid_constant__ StU U, StCoef co, int mu, int g0, Geom g) {
   int grp, p, i;
-  if (!st_block(g, 3, grp, p, i)) return;
+  if (!st_block<NG>(g, g0, grp, p, i)) return;
   const StSite s = st_site(g, i, p);
   const int r = threadIdx.y, j1 = grp == 0 ? 1 : 0, j2 = grp == 2 ? 1 : 2;
   const i64 Vh = g.Vh;
@@ -237,13 +244,14 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_chain_x(const __grid_
   }
 }
 
-// row r of c1 in + w sum_n staple(Y_n; n)
+// row r of c1 in + w sum_n staple(Y_n; n), without the n whose Y is null
 __device__ __forceinline__ void st_fat_row(const Geom &g, const StSite &s, const double2 *in,
                                            const double2 *const (&Y)[3], const StU &U, double c1, double w, int mu,
                                            int r, double2 (&a)[1][3]) {
   const i64 Vh = g.Vh;
 #pragma unroll 1
   for (int j = 0; j < 3; j++) {
+    if (!Y[j]) continue;   // uniform
     const double2 *const y[1] = {Y[j]};
     st_staple<1>(g, s, y, U.d[st_dir(mu, j)], mu, st_dir(mu, j), r, a);
   }
