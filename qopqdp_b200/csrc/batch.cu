@@ -256,8 +256,8 @@ struct BList {
 // one and stores nothing.
 template <int NL, int KIND, bool RECON, int BP, int MINB>
 __global__ void __launch_bounds__(QB, MINB)
-k_bhop_pair(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned char *__restrict__ lk,
-            const uint4 *__restrict__ same, Geom g, NbrGeom ng, int p, MixState *st, const __grid_constant__ BList bl,
+k_bhop_pair(uint4 *__restrict__ out, const uint4 *src, const unsigned char *__restrict__ lk,
+            const uint4 *same, Geom g, NbrGeom ng, int p, MixState *st, const __grid_constant__ BList bl,
             int ngrp, double *part, unsigned *count, float c_long) {
   constexpr int BG = 2 * BP;
   const int grp = blockIdx.x % ngrp, sb = blockIdx.x / ngrp, nsb = gridDim.x / ngrp;
@@ -422,7 +422,7 @@ static void launch_bhop_list(bool pdl, int nl, bool recon, int nsb, uint4 *out, 
 
 // x_j += alpha_j p_j, r_j -= alpha_j Ap_j, |r_j|^2: blockIdx.y = list entry
 __global__ void __launch_bounds__(256)
-k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *__restrict__ p, const uint4 *__restrict__ Ap,
+k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *p, const uint4 *Ap,
           i64 Vh, MixState *st, const __grid_constant__ BList bl, double *part, unsigned *count) {
   pdl_wait();
   const int j = bl.s[blockIdx.y];
@@ -464,7 +464,7 @@ k_bupdate(float2 *__restrict__ xs, uint4 *__restrict__ r, const uint4 *__restric
 
 // p_j = r_j + beta_j p_j: blockIdx.y = list entry
 __global__ void __launch_bounds__(256)
-k_bp(uint4 *__restrict__ p, const uint4 *__restrict__ r, i64 Vh, const MixState *st,
+k_bp(uint4 *__restrict__ p, const uint4 *r, i64 Vh, const MixState *st,
      const __grid_constant__ BList bl) {
   pdl_wait();
   const int j = bl.s[blockIdx.y];

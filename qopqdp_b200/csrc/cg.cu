@@ -20,7 +20,7 @@ constexpr int CG_CHUNK = 32;   // iterations per host check
 
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS)
-k_cg_update(c2<T> *__restrict__ x, c2<T> *__restrict__ r, const c2<T> *__restrict__ p, const c2<T> *__restrict__ Ap,
+k_cg_update(c2<T> *__restrict__ x, c2<T> *__restrict__ r, const c2<T> *p, const c2<T> *Ap,
             int n, CgState *st, double *part, unsigned *count) {
   pdl_wait();
   if (st->flag) return;
@@ -46,7 +46,7 @@ k_cg_update(c2<T> *__restrict__ x, c2<T> *__restrict__ r, const c2<T> *__restric
 
 template <typename T>
 __global__ void __launch_bounds__(RED_THREADS)
-k_cg_p(c2<T> *__restrict__ p, const c2<T> *__restrict__ r, int n, const CgState *st) {
+k_cg_p(c2<T> *__restrict__ p, const c2<T> *r, int n, const CgState *st) {
   pdl_wait();
   if (st->flag) return;
   const T b = (T)st->b;

@@ -82,8 +82,8 @@ __device__ __forceinline__ void hop_mul(c2<T> (&a)[3], const c2<T> (&U)[9], c2<T
 // st: solver state of a device-driven CG (cg.cuh) or null.
 template <typename T, int NL, int MODE, int RED, bool DD = false, int SPLIT = 1, bool BOTH = false>
 __global__ void __launch_bounds__(hop_threads(SPLIT), hop_minb<T>(SPLIT, DD, RED))
-k_hop(c2<T> *__restrict__ out, const c2<T> *__restrict__ src, const c2<T> *__restrict__ lk,
-      const c2<T> *__restrict__ same, T mass, Geom g, int p, int tile, double *part, unsigned *count, double *res,
+k_hop(c2<T> *__restrict__ out, const c2<T> *src, const c2<T> *__restrict__ lk,
+      const c2<T> *same, T mass, Geom g, int p, int tile, double *part, unsigned *count, double *res,
       CgState *st, DdGhost<T> gh = DdGhost<T>()) {
   static_assert(!DD || (SPLIT == 1 && !BOTH), "halo reads: one thread per site, one parity");
   constexpr int NS = NL / SPLIT, SITES = hop_sites(SPLIT);

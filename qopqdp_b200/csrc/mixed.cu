@@ -148,7 +148,7 @@ k_mix_p(typename Sp::elem *__restrict__ p, const typename Sp::elem *__restrict__
 template <class Sp>
 __global__ void __launch_bounds__(256)
 k_mix_update_p(float2 *__restrict__ xs, typename Sp::elem *__restrict__ r, typename Sp::elem *__restrict__ p,
-               const typename Sp::elem *__restrict__ Ap, i64 Vh, const MixState *st, int seq) {
+               const typename Sp::elem *Ap, i64 Vh, const MixState *st, int seq) {
   pdl_wait();
   if (st->tok != seq) return;
   const int fl = st->flag;
@@ -345,7 +345,7 @@ k_ms_p(typename Sp::elem *__restrict__ p, const typename Sp::elem *__restrict__ 
 template <class Sp>
 __global__ void __launch_bounds__(256)
 k_ms_update_fused(float2 *__restrict__ xs, typename Sp::elem *__restrict__ r, typename Sp::elem *__restrict__ p,
-                  const typename Sp::elem *__restrict__ Ap, i64 Vh, MixState *st, int seq, double *part,
+                  const typename Sp::elem *Ap, i64 Vh, MixState *st, int seq, double *part,
                   unsigned *count, MsShift *sh, int ns, MsVecs mv) {
   typedef typename Sp::elem E;
   pdl_wait();
@@ -904,9 +904,9 @@ __device__ __forceinline__ void l2_prefetch_bulk(const void *p, unsigned bytes) 
 template <int NL, int KIND, int BATCH, bool RECON, int MINB = 1, bool PERSIST = false, bool PK = false,
           bool DDQ = false, int PF = 0>
 __global__ void __launch_bounds__(QB, MINB)
-k_mix_hop_q16r(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned char *__restrict__ lk,
-               const uint4 *__restrict__ same, Geom g, NbrGeom ng, int p, MixState *st, double *part,
-               unsigned *count, float c_long, const uint4 *__restrict__ rres = nullptr, int seq = 0,
+k_mix_hop_q16r(uint4 *__restrict__ out, const uint4 *src, const unsigned char *__restrict__ lk,
+               const uint4 *same, Geom g, NbrGeom ng, int p, MixState *st, double *part,
+               unsigned *count, float c_long, const uint4 *rres = nullptr, int seq = 0,
                DdQ16Ghost gh = DdQ16Ghost()) {
   if constexpr (PK) pdl_wait();   // the packed variants may be launched as dependents
   if (st->flag) return;
@@ -1019,9 +1019,9 @@ k_mix_hop_q16r(uint4 *__restrict__ out, const uint4 *__restrict__ src, const uns
 constexpr int Q16S_SITES = 64;
 template <int NL, int KIND, bool RECON>
 __global__ void __launch_bounds__(4 * Q16S_SITES)
-k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *__restrict__ src, const unsigned char *__restrict__ lk,
-               const uint4 *__restrict__ same, Geom g, NbrGeom ng, int p, MixState *st, double *part,
-               unsigned *count, float c_long, const uint4 *__restrict__ rres, int seq) {
+k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *src, const unsigned char *__restrict__ lk,
+               const uint4 *same, Geom g, NbrGeom ng, int p, MixState *st, double *part,
+               unsigned *count, float c_long, const uint4 *rres, int seq) {
   constexpr int NS = NL / 4;
   const int t = threadIdx.x % Q16S_SITES, w = threadIdx.x / Q16S_SITES;   // w: uniform over a warp, the direction
   const i64 Vh = g.Vh;

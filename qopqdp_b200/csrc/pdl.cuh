@@ -9,6 +9,11 @@
 // or three ahead still run may read lines of their vectors that its
 // multiprocessor's L1 kept from before (seen as solves that needed a third
 // more iterations), and it gained nothing (8^4 FP32 CG 4.2 ms without, 4.4 with).
+// Vectors that a kernel ahead writes are plain pointers in these kernels:
+// `const ... *__restrict__` would let the compiler read them through the
+// read-only path and treat them as unchanging for the kernel's whole life,
+// which begins before the wait.  The links, which no kernel of a chain writes,
+// keep it, and may be read ahead of the wait.
 #pragma once
 #include "qopb.h"
 
