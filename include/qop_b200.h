@@ -37,6 +37,9 @@ int QOPB_prof_every(int n);
 
 /* Number of kernels the library has launched since it was loaded. */
 unsigned long long QOPB_launch_count(void);
+/* Of those, the ones launched as programmatic dependents of the kernel ahead
+   (option pdl; none while it is 0). */
+unsigned long long QOPB_dependent_launch_count(void);
 /* Failure injection for tests: the n-th device allocation from now on
    (n >= 1) fails as an out-of-memory would, and the call that makes it
    reports QOP_MEM_ERROR; n = 0 cancels.  Returns 0, or -1 for n < 0. */

@@ -24,6 +24,8 @@ void check_cuda(cudaError_t e, const char *what, const char *file, int line) {
 static unsigned long long g_launches = 0;
 void count_launches(int n) { g_launches += (unsigned long long)n; }
 unsigned long long launch_count() { return g_launches; }
+static unsigned long long g_dependents = 0;
+void count_dependents(int n) { g_dependents += (unsigned long long)n; }
 
 void fail(QOP_status_t s, const char *fmt, ...) {
   char buf[512];
@@ -238,6 +240,7 @@ QOP_status_t QOP_finalize(void) {
 int QOP_is_initialized(void) { return ctx().inited; }
 
 unsigned long long QOPB_launch_count(void) { return launch_count(); }
+unsigned long long QOPB_dependent_launch_count(void) { return g_dependents; }
 
 int QOPB_inject_alloc_failure(int n) {
   if (n < 0) return -1;

@@ -21,28 +21,25 @@ namespace qopb {
 
 __device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 
-// with dynamic shared memory (smem bytes)
+// pdl: as a dependent of the launch ahead, unless option pdl is 0
 template <typename... KArgs, typename... Args>
-void launch_ks(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, size_t smem, cudaStream_t s, Args... args) {
-  if (!pdl) {
-    k<<<grid, block, smem, s>>>(args...);
+void launch_k(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
+  if (!pdl || !ctx().opt.pdl) {
+    k<<<grid, block, 0, s>>>(args...);
     return;
   }
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
-  cfg.dynamicSmemBytes = smem;
+  cfg.dynamicSmemBytes = 0;
   cfg.stream = s;
   cudaLaunchAttribute at[1];
   at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   at[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = at;
   cfg.numAttrs = 1;
+  count_dependents(1);
   QCHECK(cudaLaunchKernelEx(&cfg, k, args...));
-}
-template <typename... KArgs, typename... Args>
-void launch_k(bool pdl, void (*k)(KArgs...), dim3 grid, dim3 block, cudaStream_t s, Args... args) {
-  launch_ks(pdl, k, grid, block, (size_t)0, s, args...);
 }
 
 }  // namespace qopb

@@ -42,6 +42,7 @@ void check_cuda(cudaError_t e, const char *what, const char *file, int line);
 // every kernel launch is followed by QLAUNCH (or QLAUNCHN for n launches),
 // which checks the launch and counts it (QOPB_launch_count)
 void count_launches(int n);
+void count_dependents(int n);   // of those, the programmatic dependents (QOPB_dependent_launch_count)
 #define QLAUNCHN(n) (::qopb::count_launches(n), ::qopb::check_cuda(cudaGetLastError(), "kernel launch", __FILE__, __LINE__))
 #define QLAUNCH() QLAUNCHN(1)
 [[noreturn]] void fail(QOP_status_t s, const char *fmt, ...);
@@ -117,7 +118,7 @@ struct Options {
   double ms_stop = -1;           // multi-shift phase: a shifted system (not the lightest mass) stops at max(its rsqmin, ms_stop); -1: 1e-10 with int16 storage, else 0
   int fuse_update = 1;           // int16 hop variants 20-26: 1 = the second hop reduces for a fused x / r / p update
   int batch_tail = 1;            // batched solves: 1 = the last running system finishes in the one-system solver
-  int pdl = 1;                   // fused int16 iteration: 1 = its kernels launched as programmatic dependents
+  int pdl = 1;                   // 1 = kernels that only follow the one ahead are launched as programmatic dependents (pdl.cuh)
   int serve_policy = 0;          // solve service: 0 = step every engine in turn, 1 = only the one with the oldest request
   double serve_hbm_mb = 0;       // solve service: device memory all engines together may hold (MB; 0 = free HBM less 2 GiB)
   int mbar_tries = 1 << 22;      // bounded mbarrier waits of the TMA-staged int16 hops: polls before MIX_ERROR
