@@ -12,7 +12,9 @@
 // 75.2 -> 44.5 ms).
 #include "cg.cuh"
 #include "pdl.cuh"
+#include "prof.cuh"
 #include "reduce.cuh"
+#include <vector>
 
 namespace qopb {
 
@@ -65,11 +67,14 @@ void cg_run(LinOp<T> &L, c2<T> *x, c2<T> *r, c2<T> *p, c2<T> *Ap, int eo, bool d
   s.flag = CG_RUN;
   s.done = 0;
   CgState *st = (CgState *)dmalloc(sizeof(CgState));
+  std::vector<int> mark;   // timing records before each iteration of a chunk
   try {
     QCHECK(cudaMemcpyAsync(st, &s, sizeof s, cudaMemcpyHostToDevice, c.s));
     while (s.flag == CG_RUN) {
-      const int chunk = s.left < CG_CHUNK ? s.left : CG_CHUNK;
+      const int chunk = s.left < CG_CHUNK ? s.left : CG_CHUNK, done0 = s.done;
+      mark.clear();
       for (int k = 0; k < chunk; k++) {
+        mark.push_back(prof_mark());
         Dslash<T>::cg_hops(L.f, L.mass, Ap, p, eo, L.tmp, st, dot, k == 0);
         launch_k(true, k_cg_update<T>, grid, RED_THREADS, c.s, x + q.off, r + q.off, (const c2<T> *)(p + q.off),
                  (const c2<T> *)(Ap + q.off), n, st, c.d_part, c.d_count);
@@ -80,6 +85,11 @@ void cg_run(LinOp<T> &L, c2<T> *x, c2<T> *r, c2<T> *p, c2<T> *Ap, int eo, bool d
       QCHECK(cudaMemcpyAsync(c.h_res, st, sizeof s, cudaMemcpyDeviceToHost, c.s));
       sync();
       memcpy(&s, c.h_res, sizeof s);
+      // drop timing records of hops that found the flag set (no work); a
+      // breakdown is found by an iteration that is not counted
+      const int ran = s.done - done0 + (s.flag == CG_BREAK || s.flag == CG_NAN ? 1 : 0);
+      if (ran < chunk)
+        for (int k = mark[ran], end = prof_mark(); k < end; k++) prof_discard(k);
     }
   } catch (...) {
     dfree(st);

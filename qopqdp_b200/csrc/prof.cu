@@ -65,6 +65,7 @@ void prof_discard(int idx) {
 }
 
 bool prof_active() { return g_prof.active; }
+int prof_mark() { return (int)g_prof.recs.size(); }
 
 int tune_pick(const std::vector<int> &cand, const std::function<void(int)> &launch, int reps) {
   Context &c = ctx();

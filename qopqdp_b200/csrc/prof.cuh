@@ -8,6 +8,7 @@ namespace qopb {
 int prof_start(const char *name, double bytes);   // -1 when inactive
 void prof_stop(int idx);
 void prof_discard(int idx);
+int prof_mark();   // records so far: those of the launches between two marks lie between them
 bool prof_active();
 
 // autotuner: after one warm-up launch of each candidate, times `reps`
