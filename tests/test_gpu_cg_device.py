@@ -84,7 +84,7 @@ def test_timing_classes_count_the_hops_that_ran(prec, eo):
                 assert q.invert(fla, 0.2, hout, hin, ia, ra).status == 0
             finally:
                 st = (_Kstat * 64)()
-                n = q.lib.QOPB_prof_end(st, 64)
+                n = q.lib["QOPB_prof_end"](st, 64)   # an entry of its own, without argtypes
                 q.lib.QOP_verbose(old)
             hops = {st[k].name: st[k].launches for k in range(n) if st[k].name.startswith(b"hop_")}
             seen[verbose] = (ra.final_iter, hops)
