@@ -280,16 +280,25 @@ constexpr int HOP_BLOCK = 128;
 // thread
 template <typename T> constexpr int hop_split() { return sizeof(T) == 4 ? 4 : 8; }
 // Where the split pays (us per call through the C ABI, split / one thread per
-// site; Vh = sites per parity).  One parity: FP32 always (8^4 17 / 24,
-// Vh 80000 28 / 40, 24^3x48 77 / 87, 32^3x64 209 / 216), FP64 up to 210000
-// (80000 46 / 57, 166000 75 / 78, 207000 91 / 111; 249000 105 / 106, 332000
-// 134-194 / 144: the eight partial rows cost more than the latency they hide
-// once HBM is busy).  Both parities: the neighbours' links are read through
-// L2 as often, and the line lies lower: 10400 20 / 24 (FP32), 23 / 26 (FP64);
-// 32800 26 / 25 and 37 / 34.
-template <typename T> static bool use_split(i64 Vh, bool both) {
+// site; Vh = sites per parity).
+// One parity without a reduction: FP32 always (Vh 2048 16 / 24, 32768 17 / 23,
+// 80000 25 / 35, 165888 44 / 51, 221184 53 / 57, 331776 80 / 94, 1048576
+// 216 / 224), FP64 up to 210000 (2048 13 / 20, 32768 20 / 22, 65536 37 / 43,
+// 165888 71 / 87; 249000 105 / 106, 331776 134-194 / 144: the eight partial
+// rows cost more than the latency they hide once HBM is busy).
+// With a reduction the blocks of 32 sites leave four times as many partial
+// sums to the last block, and the line lies lower.  Operator with norm, and
+// one CG iteration: FP32 65536 70 / 106 and 66 / 96, 80000 82 / 107 and
+// 78 / 99, 120960 108 / 110 and 111 / 108, 165888 144 / 119 and 144 / 117,
+// 1048576 772 / 536; FP64 32768 66 / 107 and 59 / 97, 65536 97 / 114 and
+// 102 / 109, 80000 117 / 119 and 120 / 115, 120960 157 / 133 and 169 / 135,
+// 165888 206 / 156 and 221 / 161.
+// Both parities: the neighbours' links are read through L2 as often: 10400
+// 20 / 24 (FP32), 23 / 26 (FP64); 32800 26 / 25 and 37 / 34.
+template <typename T> static bool use_split(i64 Vh, bool both, bool red) {
   if (both) return Vh <= 20000;
-  return Vh <= (sizeof(T) == 4 ? 130000 : 210000);
+  if (red) return Vh <= (sizeof(T) == 4 ? 110000 : 75000);
+  return sizeof(T) == 4 || Vh <= 210000;
 }
 
 // x1 coordinates per tile of a two-parity hop: the forward links of the four
@@ -342,14 +351,14 @@ static void launch_hop(FlaT<T> *f, c2<T> *out, const c2<T> *in, const c2<T> *sam
     }
   }
   ProfScope ps(sizeof(T) == 8 ? "hop_f64" : "hop_f32", bytes);
-  constexpr int S = hop_split<T>();
+  constexpr int S = hop_split<T>(), ONE = sizeof(T) == 4 && RED == 0 ? S : 1;   // without a reduction FP32 is always split
 #define HOP_ARGS pdl, o, src, lk, sm, mass, p, res, st, c.d_part, c.d_count
-  if (use_split<T>(g.Vh, false)) {
+  if (use_split<T>(g.Vh, false, RED != 0)) {
     if (f->nlinks == 16) launch_hop_s<T, 16, MODE, RED, S>(HOP_ARGS);
     else launch_hop_s<T, 8, MODE, RED, S>(HOP_ARGS);
   } else {
-    if (f->nlinks == 16) launch_hop_s<T, 16, MODE, RED, 1>(HOP_ARGS);
-    else launch_hop_s<T, 8, MODE, RED, 1>(HOP_ARGS);
+    if (f->nlinks == 16) launch_hop_s<T, 16, MODE, RED, ONE>(HOP_ARGS);
+    else launch_hop_s<T, 8, MODE, RED, ONE>(HOP_ARGS);
   }
 #undef HOP_ARGS
   QLAUNCH();
@@ -361,7 +370,7 @@ static void launch_hop_both(FlaT<T> *f, c2<T> *out, const c2<T> *in, const c2<T>
   Context &c = ctx();
   const Geom &g = c.g;
   const int tile = hop_tile<T>(g, f->nlinks);
-  const bool split = use_split<T>(g.Vh, true);
+  const bool split = use_split<T>(g.Vh, true, false);
   const int sites = hop_sites(split ? 4 : 1);
   const i64 plane = g.L[2] * g.L[3] / 2, full = g.L[1] / tile, last = g.L[1] - full * tile;
   const i64 blocks = 2 * g.L[0] * (full * ((tile * plane + sites - 1) / sites) + (last * plane + sites - 1) / sites);

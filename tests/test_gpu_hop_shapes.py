@@ -1,7 +1,9 @@
 """The hop kernels at the shapes their dispatch depends on, against the
 oracle: site counts that do not fill a block (6x6x6x10: 1080 sites per
-parity, blocks of 32 and 64), the smallest extents, and a lattice whose
-two-parity FP64 hop walks x1 in two unequal tiles."""
+parity, blocks of 32 and 64), the smallest extents, a lattice whose
+two-parity FP64 hop walks x1 in two unequal tiles, and one (10x22x26x50:
+143000 sites per parity) on which the slots of a site are spread over warps
+without a reduction and not with one."""
 import itertools
 
 import numpy as np
@@ -28,7 +30,7 @@ def _setup(L, prec, naik):
 
 @pytest.mark.parametrize("prec", ["D", "F"])
 @pytest.mark.parametrize("L,naik", [((4, 4, 4, 4), True), ((6, 6, 6, 10), True), ((6, 6, 6, 10), False),
-                                    ((6, 24, 24, 34), True)])
+                                    ((6, 24, 24, 34), True), ((10, 22, 26, 50), True), ((10, 22, 26, 50), False)])
 def test_hop_shapes(prec, L, naik):
     q, fla, fo = _setup(L, prec, naik)
     V = int(np.prod(L))
