@@ -1089,11 +1089,12 @@ k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *src, const unsigned char *_
   else q16_finish<1>(acc, part, count, st);
 }
 
-// The split hops take the default variant's place between the smallest size
-// that was timed and the one where HBM and issue take over from latency (ms per
-// solve, split / general: 8^4 13.3 / 15.7, 12^4 14.6 / 17.3, 16^4 20.1 / 22.2,
-// 16^3x32 30.5 / 28.8, 20^4 36.5 / 31.5).
-static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh >= 2048 && Vh <= 32768; }
+// The split hops take the place of variant 25 (the default) up to the size
+// where HBM and issue take over from latency (ms per HISQ solve, split /
+// general: 4^4 11.1 / 13.0, 4^3x8 11.8 / 13.8, 6^4 12.7 / 14.6, 8^4 13.3 / 14.8,
+// 12^4 14.7 / 16.7, 16^4 20.6 / 23.1, 16^3x20 23.6 / 24.6, 16^3x24 25.4 / 25.4,
+// 16^3x32 30.4 / 28.6).
+static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh <= 45000; }
 
 template <int KIND>
 static void launch_q16_small(int nl, bool recon, float c_long, uint4 *out, const uint4 *src, const unsigned char *lk,
@@ -1517,7 +1518,7 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
   const bool fuse = q16v && c.opt.fuse_update && hk >= 20;
   // the three kernels of the fused iteration as programmatic dependents
   const bool pdl = fuse && c.opt.pdl;
-  // the default hop on a small lattice (the numbered variants keep their shapes)
+  // variant 25 on a small lattice (the other numbers keep their shapes everywhere)
   const bool small = fuse && !dd_active() && use_q16_small(Vh);
   int seq = 0;
   // a decomposed lattice: halos before each hop, the reductions summed over

@@ -29,7 +29,8 @@ def _links(L, kind):
     return fat, lng, geo, dbl, dq
 
 
-@pytest.mark.parametrize("L", [(8, 8, 8, 8), (6, 6, 10, 14)])
+@pytest.mark.parametrize("L", [(4, 4, 4, 4), (4, 4, 4, 6), (6, 6, 6, 10), (8, 8, 8, 8), (6, 6, 10, 14),
+                               (16, 16, 16, 20), (16, 16, 18, 20)])   # the last on the general hop
 @pytest.mark.parametrize("kind", ["hisq", "general"])
 @pytest.mark.parametrize("eo", [0, 1])
 def test_split_hop(L, kind, eo):
