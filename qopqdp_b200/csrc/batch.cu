@@ -499,6 +499,7 @@ struct BhopShape { int bg, minb; };
 static const BhopShape kBhop[] = {{4, 1}, {4, 5}, {2, 8}, {2, 1}, {8, 1}, {4, 6}, {4, 5}, {8, 3}, {8, 2},
                                   {8, 3}, {8, 4}, {16, 2}, {4, 5}, {8, 3}, {8, 2}, {4, 4}};
 constexpr int N_BHOP = (int)(sizeof(kBhop) / sizeof(kBhop[0]));
+constexpr int BHOP_LIST = -1;   // the list hop (k_bhop_pair)
 
 template <int KIND, int BG, int MINB, int UNR = 16, bool PK = false>
 static void launch_bhop_t(int nl, bool recon, int ngrp, int nsb, uint4 *out, const uint4 *src,
@@ -800,8 +801,8 @@ void BatchEngine::launch() {
   const float c_long = (float)sl->c_long;
   const int nsb = e.nsb, gridv = e.gridv;
   QCHECK(cudaMemcpyAsync(e.dst, e.h, sizeof(MixState) * n, cudaMemcpyHostToDevice, c.s));
-  // batch_kernel -1: the list hop (k_bhop_pair); -2: the fastest of 1, 6, 7, 9, 12 timed on the first step
-  // with this lattice and number of systems
+  // batch_kernel -1: the list hop (k_bhop_pair); -2: the fastest of it and of
+  // 1, 6, 7, 9, 12, timed on the first step with this lattice and number of systems
   const double link_site = recon ? (nl / 2) * (40.0 + 28.0) : nl * 40.0;
   const int chunk = c.opt.chunk;
   std::vector<int> recs;
@@ -835,7 +836,12 @@ void BatchEngine::launch() {
     e.inflight = true;
     return;
   }
-  int variant = c.opt.batch_kernel == -1 ? 1 : std::min(c.opt.batch_kernel, N_BHOP - 1);
+  // the list hop takes the running systems from a list; the numbered variants
+  // walk all slots
+  BList bl{};
+  for (int j = 0; j < n; j++)
+    if (e.sys[j].busy && e.h[j].flag != MIX_DONE) bl.s[bl.n++] = j;
+  int variant = std::min(c.opt.batch_kernel, N_BHOP - 1);
   if (c.opt.batch_kernel == -2) {
     const std::array<int, 7> key{g.L[0], g.L[1], g.L[2], g.L[3], nl, recon ? 1 : 0, n};
     auto it = g_bhop_tuned.find(key);
@@ -843,24 +849,22 @@ void BatchEngine::launch() {
       variant = it->second;
     } else {
       const unsigned char *lq = (const unsigned char *)lk_q.a;
-      variant = tune_pick({1, 6, 7, 9, 12}, [&](int v) {   // t = D p: recomputed by the first iteration
-        launch_bhop<1>(v, nl, recon, (n + kBhop[v].bg - 1) / kBhop[v].bg, nsb, e.ts, e.ps, lq, nullptr, g, e.ng, q,
-                       e.dst, n, e.part, e.count, c_long);
+      char what[40];
+      snprintf(what, sizeof what, "batched hop of %d systems", n);
+      variant = tune_pick(what, {BHOP_LIST, 1, 6, 7, 9, 12}, [&](int v) {   // t = D p: recomputed by the first iteration
+        if (v == BHOP_LIST)
+          launch_bhop_list<1>(false, nl, recon, nsb, e.ts, e.ps, lq, nullptr, g, e.ng, q, e.dst, bl, e.part, e.count,
+                              c_long);
+        else
+          launch_bhop<1>(v, nl, recon, (n + kBhop[v].bg - 1) / kBhop[v].bg, nsb, e.ts, e.ps, lq, nullptr, g, e.ng, q,
+                         e.dst, n, e.part, e.count, c_long);
         QLAUNCH();
       });
       g_bhop_tuned[key] = variant;
-      log0(QOP_VERB_LOW, "autotune: batched hop variant %d for %d systems on %dx%dx%dx%d\n", variant, n, g.L[0],
-           g.L[1], g.L[2], g.L[3]);
     }
   }
-  // the default hop takes the running systems from a list (k_bhop_pair); the
-  // numbered variants walk all slots
-  const bool ab = c.opt.batch_kernel == -1;
-  BList bl{};
-  for (int j = 0; j < n; j++)
-    if (e.sys[j].busy && e.h[j].flag != MIX_DONE) bl.s[bl.n++] = j;
-  const int BG = kBhop[variant].bg;
-  const int ngrp = (n + BG - 1) / BG;
+  const bool ab = variant == BHOP_LIST;
+  const int ngrp = ab ? 0 : (n + kBhop[variant].bg - 1) / kBhop[variant].bg;   // of a numbered variant
   char hname[32];
   snprintf(hname, sizeof hname, "bhop_q16_x%d", active);   // timing class: systems running in the launch
   // compulsory bytes of one hop for the systems running in this chunk

@@ -1094,6 +1094,7 @@ k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *src, const unsigned char *_
 // general: 4^4 11.1 / 13.0, 4^3x8 11.8 / 13.8, 6^4 12.7 / 14.6, 8^4 13.3 / 14.8,
 // 12^4 14.7 / 16.7, 16^4 20.6 / 23.1, 16^3x20 23.6 / 24.6, 16^3x24 25.4 / 25.4,
 // 16^3x32 30.4 / 28.6).
+constexpr int HOP_SMALL = 32;   // the split hops in the tuner's list: no value of the option
 static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh <= 45000; }
 
 template <int KIND>
@@ -1393,8 +1394,8 @@ struct MsArgs {
 };
 
 // autotuned int16 hop variant per (lattice extents, links per site, long-link
-// reconstruction)
-static std::map<std::array<int, 6>, int> g_hop_tuned;
+// reconstruction, fused update)
+static std::map<std::array<int, 7>, int> g_hop_tuned;
 
 template <class Sp, class Lk>
 static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *ra, c2<double> *x,
@@ -1494,11 +1495,13 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
   // update needs and one kernel updates x, r and p
   constexpr bool q16v = std::is_same<Lk, LkQ16B>::value && std::is_same<Sp, SpQ16>::value;
   // int16 hop variant: the option, or (hop_kernel -1) the fastest of the
-  // packed persistent variants 20-26 timed on this lattice's first solve
+  // packed persistent variants 20-26 and, with the fused update, the split hop
+  // timed on this lattice's first solve
   int hk = c.opt.hop_kernel;
   if constexpr (std::is_same<Lk, LkQ16B>::value) {
     if (hk < 0) {
-      const std::array<int, 6> key{g.L[0], g.L[1], g.L[2], g.L[3], nl, recon ? 1 : 0};
+      const bool spl = q16v && c.opt.fuse_update;
+      const std::array<int, 7> key{g.L[0], g.L[1], g.L[2], g.L[3], nl, recon ? 1 : 0, spl ? 1 : 0};
       auto it = g_hop_tuned.find(key);
       if (dd_active()) {
         hk = 25;   // the decomposed hop has the shape of variant 25
@@ -1506,12 +1509,19 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
         hk = it->second;
       } else {
         const unsigned char *lq = (const unsigned char *)lk_q.a;
-        hk = tune_pick({20, 21, 22, 23, 24, 25, 26}, [&](int v) {   // t = D p: recomputed by the first iteration
-          launch_q16<1>(v, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst);
+        std::vector<int> cand{20, 21, 22, 23, 24, 25, 26};
+        if (spl) cand.push_back(HOP_SMALL);
+        hk = tune_pick("int16 hop", cand, [&](int v) {   // t = D p: recomputed by the first iteration
+          if constexpr (q16v) {
+            if (v == HOP_SMALL)
+              launch_q16_small<1>(nl, recon, c_long, ts, ps, lq, nullptr, g, ng, q, dst, nullptr, 0, false);
+            else launch_q16<1>(v, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst);
+          } else {
+            launch_q16<1>(v, nl, recon, c_long, gridq, ts, ps, lq, nullptr, g, ng, q, dst);
+          }
           QLAUNCH();
         });
         g_hop_tuned[key] = hk;
-        log0(QOP_VERB_LOW, "autotune: int16 hop variant %d on %dx%dx%dx%d\n", hk, g.L[0], g.L[1], g.L[2], g.L[3]);
       }
     }
   }
@@ -1519,7 +1529,7 @@ static void run_mixed(LinOp<double> &L, QOP_invert_arg_t *ia, QOP_resid_arg_t *r
   // the three kernels of the fused iteration as programmatic dependents
   const bool pdl = fuse && c.opt.pdl;
   // variant 25 on a small lattice (the other numbers keep their shapes everywhere)
-  const bool small = fuse && !dd_active() && use_q16_small(Vh);
+  const bool small = fuse && !dd_active() && (hk == HOP_SMALL || use_q16_small(Vh));
   int seq = 0;
   // a decomposed lattice: halos before each hop, the reductions summed over
   // the processes before the scalars (the fused int16 iteration only)

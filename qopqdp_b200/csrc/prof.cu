@@ -67,8 +67,9 @@ void prof_discard(int idx) {
 bool prof_active() { return g_prof.active; }
 int prof_mark() { return (int)g_prof.recs.size(); }
 
-int tune_pick(const std::vector<int> &cand, const std::function<void(int)> &launch, int reps) {
+int tune_pick(const char *what, const std::vector<int> &cand, const std::function<void(int)> &launch, int reps) {
   Context &c = ctx();
+  std::string times;
   cudaEvent_t a = nullptr, b = nullptr;
   int best = cand.empty() ? -1 : cand[0];
   float best_ms = 3.0e38f;
@@ -84,6 +85,9 @@ int tune_pick(const std::vector<int> &cand, const std::function<void(int)> &laun
       float ms = 0;
       QCHECK(cudaEventElapsedTime(&ms, a, b));
       if (ms < best_ms) { best_ms = ms; best = v; }
+      char t[48];
+      snprintf(t, sizeof t, " %d (%.1f us)", v, 1e3 * ms / reps);
+      times += t;
     }
   } catch (...) {
     if (a) cudaEventDestroy(a);
@@ -92,6 +96,8 @@ int tune_pick(const std::vector<int> &cand, const std::function<void(int)> &laun
   }
   cudaEventDestroy(a);
   cudaEventDestroy(b);
+  log0(QOP_VERB_LOW, "autotune: %s on %dx%dx%dx%d:%s, taken %d\n", what, c.g.L[0], c.g.L[1], c.g.L[2], c.g.L[3],
+       times.c_str(), best);
   return best;
 }
 

@@ -14,8 +14,9 @@ bool prof_active();
 // autotuner: after one warm-up launch of each candidate, times `reps`
 // launches of it with CUDA events on the library stream and returns the
 // candidate with the least time.  launch(v) must be idempotent (its outputs
-// are recomputed by the caller's next real launch).
-int tune_pick(const std::vector<int> &cand, const std::function<void(int)> &launch, int reps = 3);
+// are recomputed by the caller's next real launch).  `what` names the choice
+// in the line that QOP_VERB_LOW prints with every candidate's time.
+int tune_pick(const char *what, const std::vector<int> &cand, const std::function<void(int)> &launch, int reps = 3);
 
 struct ProfScope {
   int idx;

@@ -346,10 +346,40 @@ def test_every_batch_kernel_variant():
     q.destroy_L(fla)
 
 
+def test_autotuners_time_the_default_hops(capfd):
+    """The candidates of hop_kernel -1 and batch_kernel -2 include the hops
+    that the defaults take: the split hop of small lattices (32 in the list;
+    with the fused update only) and the list hop (-1)."""
+    L = (4, 4, 6, 10)   # no other test tunes on it
+    q = gpu_lattice(L, "D")
+    fat, lng = asqtad_links(L, 0.3, 7)
+    fla = q.create_L_from_raw(fat, lng)
+    srcs = [LT.gaussian_vector(L, 340 + s) for s in range(3)]
+    old = q.lib.QOP_verbose(1)
+    try:
+        said = {}
+        for fuse in (1, 0):
+            assert q.set_opts(prec_sloppy=16, hop_kernel=-1, batch_kernel=-2, fuse_update=fuse) == 0
+            capfd.readouterr()
+            assert _single_iters(q, fla, srcs[0], 0.1, L)[0] == 0
+            if fuse:
+                assert _run_multi(q, fla, [[0.1]] * 3, srcs, 1e-16)[0].status == 0
+            said[fuse] = [l for l in capfd.readouterr().out.splitlines() if l.startswith("autotune: ")]
+    finally:
+        q.lib.QOP_verbose(old)
+        assert q.set_opts(prec_sloppy=64, hop_kernel=25, batch_kernel=-1, fuse_update=1) == 0
+    hop = [[l for l in said[f] if "int16 hop" in l] for f in (0, 1)]
+    assert len(hop[0]) == len(hop[1]) == 1, said
+    assert " 25 (" in hop[1][0] and " 32 (" in hop[1][0] and " 32 (" not in hop[0][0], hop
+    batch = [l for l in said[1] if "batched hop of 3" in l]
+    assert len(batch) == 1 and " -1 (" in batch[0] and " 12 (" in batch[0], said
+    q.destroy_L(fla)
+
+
 def test_autotuned_hop_variants():
     """Options hop_kernel -1 and batch_kernel -2: the first solve on a
-    lattice times the candidate variants (one-system hops 20-26; batched
-    hops 1, 6, 7, 9, 12) and keeps the fastest; the solves reach the FP64
+    lattice times the candidate variants (one-system hops 20-26 and the split
+    hop; batched hops -1, 1, 6, 7, 9, 12) and keeps the fastest; the solves reach the FP64
     target with the iteration counts of the fixed defaults, and a second
     solve (cached choice) repeats the first."""
     L = (8, 8, 8, 8)
