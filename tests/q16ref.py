@@ -11,7 +11,7 @@ and the rounding of the output to int16.
 
 Links follow the reference's double-stored order (lib/asqtad_dslash_p.c:79-133):
 slot 4 mu + {fat fwd, long fwd, fat bck, long bck} with displacements
-{+1, +3, -1, -3} along mu, every link times 1/2 (:201-206), a backward link
+{+1, +3, -1, -3} along mu (2 mu + {fwd, bck} without Naik links), every link times 1/2 (:201-206), a backward link
 bck(x) = -fwd(x - d mu)^+.  Vectors are raw arrays (V, 3, 2) in the
 reference's raw site order (lib/layout_user.c:237-258).
 """
@@ -40,16 +40,21 @@ class Geometry:
                 y[:, mu] = (y[:, mu] + d) % L[mu]
                 self.nbr[(mu, d)] = LT.raw_index(L, y)
 
-    def slots(self):
-        """(mu, displacement) of the 16 double-stored slots."""
+    def slots(self, n=16):
+        """(mu, displacement) of the 16 (8 without Naik links) double-stored slots."""
+        if n == 8:
+            return [(k // 2, (1, -1)[k % 2]) for k in range(8)]
         return [(k // 4, (1, 3, -1, -3)[k % 4]) for k in range(16)]
 
 
 def dbl_links(geo, fat, lng):
-    """16 complex (V, 3, 3) arrays: the double-stored links times 1/2."""
+    """16 (8 without Naik links) complex (V, 3, 3) arrays: the double-stored links times 1/2."""
     out = []
     for mu in range(4):
         f = 0.5 * cplx(fat[mu])
+        if lng is None:
+            out += [f, -np.conj(np.swapaxes(f[geo.nbr[(mu, -1)]], 1, 2))]
+            continue
         l = 0.5 * cplx(lng[mu])
         out += [f, l,
                 -np.conj(np.swapaxes(f[geo.nbr[(mu, -1)]], 1, 2)),
@@ -104,9 +109,8 @@ def _recon_ok(longs):
 
 
 def quantize_links(dbl):
-    """the int16 link copy as decoded by the hop: 16 complex (V, 3, 3) arrays."""
-    longs = [dbl[k] for k in range(1, 16, 2)]
-    recon, c_long = _recon_ok(longs)
+    """the int16 link copy as decoded by the hop: 16 (or 8) complex (V, 3, 3) arrays."""
+    recon, c_long = _recon_ok([dbl[k] for k in range(1, 16, 2)]) if len(dbl) == 16 else (False, 0.0)
     out = []
     for k, u in enumerate(dbl):
         if recon and k % 2 == 1:
@@ -131,7 +135,7 @@ def hop(geo, links, v, sites):
     """(sum_k U_k(x) v(x + d_k mu_k), sum_k |U_k(x)|_F |v(x + d_k mu_k)|) for raw sites `sites`."""
     acc = np.zeros((len(sites), 3), dtype=np.complex128)
     mag = np.zeros(len(sites))
-    for k, (mu, d) in enumerate(geo.slots()):
+    for k, (mu, d) in enumerate(geo.slots(len(links))):
         w = v[geo.nbr[(mu, d)][sites]]
         u = links[k][sites]
         acc += np.einsum("vab,vb->va", u, w)

@@ -319,8 +319,9 @@ def test_programmatic_dependent_launch_solves_like_the_default():
 
 
 def test_every_batch_kernel_variant():
-    """Each selectable batched hop (option batch_kernel 0-15 on int16 vectors,
-    16 the tensor-core hop on bf16 hi / lo vectors) solves a four-source
+    """Each selectable batched hop (option batch_kernel -1, the default list
+    hop, and 0-15 on int16 vectors, 16 the tensor-core hop on bf16 hi / lo
+    vectors) solves a four-source
     batch to the FP64 target with the iteration counts of the default
     variant."""
     L = (8, 8, 8, 8)
@@ -331,7 +332,7 @@ def test_every_batch_kernel_variant():
     srcs = [LT.gaussian_vector(L, 340 + s) for s in range(4)]
     ms = [[0.03], [0.05], [0.03], [0.1]]
     its = {}
-    for v in range(17):
+    for v in range(-1, 17):
         assert q.set_opts(prec_sloppy=16, batch_kernel=v) == 0
         info, ras, outs = _run_multi(q, fla, ms, srcs, 1e-20)
         assert info.status == 0
@@ -342,7 +343,7 @@ def test_every_batch_kernel_variant():
     assert q.set_opts(prec_sloppy=64, batch_kernel=-1) == 0
     print("batched iterations per variant", its)
     for v, it in its.items():
-        assert all(abs(a - b) <= 0.03 * b + 3 for a, b in zip(it, its[7])), its
+        assert all(abs(a - b) <= 0.03 * b + 3 for a, b in zip(it, its[-1])), its
     q.destroy_L(fla)
 
 

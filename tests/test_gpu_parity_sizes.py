@@ -11,8 +11,8 @@
   values the device stores (tests/q16ref.py), with the bound stated there:
   |got - ref| <= 4e-5 |ref| + 1e-6 sum_k |U_k| |v_k| per site.  The norm-wise
   distance to the unquantised FP64 operator is checked too (<= 2^-12).
-* The 16-system batched hop (default 8 systems per thread) and the 12-system
-  shape (4 per thread) on the same lattice, system by system, and the
+* The default batched hop with 16 systems (two groups of 8) and with 12
+  (three of 4) on the same lattice, system by system, and the
   tensor-core hop (batch_kernel 16: mma.sync on bf16 hi / lo operands) with
   16, 12 and 3 systems against the same FP64 operator on its own storage.
 """

@@ -1,8 +1,9 @@
 """The int16 operators at the sizes where their dispatch changes, against the
 values of the stored records (tests/q16ref.py, with the per-site bounds of
 tests/test_gpu_parity_sizes.py): the split hop of small lattices with a
-partly filled last block, links with and without the rebuilt third row, and
-the batched hop for every number of systems in a group."""
+partly filled last block, links with and without the rebuilt third row and
+without Naik terms, and the batched hop for every number of systems in a
+group."""
 import numpy as np
 import pytest
 
@@ -19,19 +20,19 @@ def _links(L, kind):
     if kind == "hisq":
         fat, lng, _, _ = hisq_links(L, 0.5, 9)
     else:
-        fat, lng = asqtad_links(L, 0.3, 7)
+        fat, lng = asqtad_links(L, 0.3, 7, kind != "fat")
     if kind == "general":   # long links that are not |c| x unitary keep all three rows
         lng = tuple(a * (1 + 0.1 * np.arange(3).reshape(1, 3, 1, 1)) for a in lng)
     geo = R.Geometry(L)
     dbl = R.dbl_links(geo, fat, lng)
     dq, recon = R.quantize_links(dbl)
-    assert recon == (kind != "general")
+    assert recon == (kind == "hisq")
     return fat, lng, geo, dbl, dq
 
 
 @pytest.mark.parametrize("L", [(4, 4, 4, 4), (4, 4, 4, 6), (6, 6, 6, 10), (8, 8, 8, 8), (6, 6, 10, 14),
                                (16, 16, 16, 20), (16, 16, 18, 20)])   # the last on the general hop
-@pytest.mark.parametrize("kind", ["hisq", "general"])
+@pytest.mark.parametrize("kind", ["hisq", "general", "fat"])
 @pytest.mark.parametrize("eo", [0, 1])
 def test_split_hop(L, kind, eo):
     fat, lng, geo, dbl, dq = _links(L, kind)
@@ -53,10 +54,11 @@ def test_split_hop(L, kind, eo):
     q.destroy_L(fla)
 
 
-@pytest.mark.parametrize("n", list(range(1, 17)))
-def test_batched_hop_groups(n):
+@pytest.mark.parametrize("kind,n", [("hisq", n) for n in range(1, 17)] +
+                         [(k, n) for k in ("general", "fat") for n in (1, 3, 5, 8, 11, 16)])   # every instance
+def test_batched_hop_groups(kind, n):
     L = (6, 6, 6, 10)
-    fat, lng, geo, dbl, dq = _links(L, "hisq")
+    fat, lng, geo, dbl, dq = _links(L, kind)
     q = gpu_lattice(L, "D")
     fla = q.create_L_from_raw(fat, lng)
     masses = [0.05 * (1.2 ** j) for j in range(n)]
