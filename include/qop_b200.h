@@ -42,7 +42,8 @@ unsigned long long QOPB_launch_count(void);
 unsigned long long QOPB_dependent_launch_count(void);
 /* Failure injection for tests: the n-th device allocation from now on
    (n >= 1) fails as an out-of-memory would, and the call that makes it
-   reports QOP_MEM_ERROR; n = 0 cancels.  Returns 0, or -1 for n < 0. */
+   reports QOP_MEM_ERROR (the link and asqtad force calls try a smaller
+   workspace first); n = 0 cancels.  Returns 0, or -1 for n < 0. */
 int QOPB_inject_alloc_failure(int n);
 
 /* QOP_D3_asqtad_ddagd_norm2 without any device allocation (no counterpart

@@ -246,19 +246,21 @@ struct BList {
 // real and imaginary part in the lanes) and 8 systems share one decode of a
 // link.  Per pair of systems and slot: two 16-byte loads, 12 byte permutes,
 // 6 packed adds and 9 packed multiplies for the decode and 36 packed FMAs.
-// Latency and instruction issue bound it (a packed FMA takes two cycles of the
-// FP32 pipe; with the parts of one system in the lanes it issued at 51 % with
-// 16 warps per SM).  us per hop by running systems at 24^3x48 (variants 1 / 7
-// before): 16 242 (270), 13 256 (257), 12 215 (242), 9 201 (206), 7 150 (168),
-// 6 125 (166), 4 96 (139), 3 94 (134), 2 66 (127); 32^4, 16 sources, m 0.05:
-// the call 857 ms (1016).  A ring of cp.async stages in shared memory gained
-// less (252 us with 16) than it cost to order its refills.  A lane without a system of its own repeats the group's first
-// one and stores nothing.
+// Latency and the FP32 pipe bound it (24^4, 16 systems, first / second hop:
+// FMA pipe 59 / 55 % busy, as a packed FMA takes two of its cycles, issue
+// 53 / 50 %, DRAM 13 / 16 %; 57 / 60 instructions per system, slot and warp;
+// stalls per issue: long scoreboard 1.6 / 2.9, math pipe 1.2 / 0.8, with 15
+// warps active per SM).  us per hop by running systems at 24^3x48 (variants 1
+// / 7 before): 16 242 (270), 13 256 (257), 12 215 (242), 9 201 (206), 7 150
+// (168), 6 125 (166), 4 96 (139), 3 94 (134), 2 66 (127); 32^4, 16 sources, m
+// 0.05: the call 857 ms (1016).  A ring of cp.async stages in shared memory
+// gained less (252 us with 16) than it cost to order its refills.  A lane
+// without a system of its own repeats the group's first one and stores nothing.
 template <int NL, int KIND, bool RECON, int BP, int MINB>
 __global__ void __launch_bounds__(QB, MINB)
-k_bhop_pair(uint4 *__restrict__ out, const uint4 *src, const unsigned char *__restrict__ lk,
-            const uint4 *same, Geom g, NbrGeom ng, int p, MixState *st, const __grid_constant__ BList bl,
-            int ngrp, double *part, unsigned *count, float c_long) {
+k_bhop_pair(uint4 *__restrict__ out, const uint4 *src, const unsigned char *__restrict__ lk, const uint4 *same,
+            Geom g, NbrGeom ng, int p, MixState *st, const __grid_constant__ BList bl, int ngrp, double *part,
+            unsigned *count, float c_long) {
   constexpr int BG = 2 * BP;
   const int grp = blockIdx.x % ngrp, sb = blockIdx.x / ngrp, nsb = gridDim.x / ngrp;
   const int tid = threadIdx.x;

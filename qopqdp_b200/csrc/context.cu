@@ -144,7 +144,8 @@ static bool make_geom(const int *ls, Geom &g, bool global = false) {
   return true;
 }
 
-// fused reductions run one block per 64+ sites with up to 4 sums each
+// partial sums of one reduction over a parity: at most three a block of 64
+// sites (the fused int16 hop) or one a block of 32 (the split hops)
 static void ensure_partials(const Geom &g) {
   Context &c = g_ctx;
   size_t need = (size_t)4 * (g.Vh / 64 + 64);

@@ -69,22 +69,26 @@ __device__ __forceinline__ void hop_mul(c2<T> (&a)[3], const c2<T> (&U)[9], c2<T
 
 // RED: 0 none, 1 = sum |out|^2, 2 = sum |same|^2, 3 = Re <same, out>; DD:
 // read halos (dd.cuh).
-// SPLIT > 1 (small lattices): the slots of a site are spread over SPLIT
+// SPLIT > 1 (where use_split says): the slots of a site are spread over SPLIT
 // warps, which load their links before they wait for the kernel ahead (links
 // are never written by it: the first kernel of a dependent chain is an
-// ordinary launch), so a hop costs one round trip to L2 instead of one per
-// slot; the partial sums meet in shared memory and are added in FP64.
+// ordinary launch), so a hop costs one round trip for the links instead of
+// one per slot; the partial sums meet in shared memory and are added in FP64.
+// On lattices beyond L2 HBM bounds it: FP32, 24^3x48, one parity, reads
+// 392 MB where 390 are compulsory, at 6.1 TB/s.
 // BOTH: both parities in one launch, site blocks of the two parities next to
 // each other, and every link read as a forward link: a backward slot takes
 // the neighbour's forward link, which the neighbour's own block has brought
 // into L2.  Blocks walk the lattice in tiles of `tile` x1 coordinates so
-// that the links of the few x0 slices between the two reads stay in L2.
+// that the links of the few x0 slices between the two reads stay in L2.  HBM
+// bounds it, the part of the second reads that misses L2 included: FP64,
+// 24^3x48 reads 971 MB where 796 are compulsory, 16x32x32x64 1624 where 1258
+// are, both at 6.0-6.4 TB/s with the writes.
 // st: solver state of a device-driven CG (cg.cuh) or null.
 template <typename T, int NL, int MODE, int RED, bool DD = false, int SPLIT = 1, bool BOTH = false>
 __global__ void __launch_bounds__(hop_threads(SPLIT), hop_minb<T>(SPLIT, DD, RED))
-k_hop(c2<T> *__restrict__ out, const c2<T> *src, const c2<T> *__restrict__ lk,
-      const c2<T> *same, T mass, Geom g, int p, int tile, double *part, unsigned *count, double *res,
-      CgState *st, DdGhost<T> gh = DdGhost<T>()) {
+k_hop(c2<T> *__restrict__ out, const c2<T> *src, const c2<T> *__restrict__ lk, const c2<T> *same, T mass, Geom g,
+      int p, int tile, double *part, unsigned *count, double *res, CgState *st, DdGhost<T> gh = DdGhost<T>()) {
   static_assert(!DD || (SPLIT == 1 && !BOTH), "halo reads: one thread per site, one parity");
   constexpr int NS = NL / SPLIT, SITES = hop_sites(SPLIT);
   const i64 Vh = g.Vh;
@@ -378,7 +382,9 @@ static void launch_hop_both(FlaT<T> *f, c2<T> *out, const c2<T> *in, const c2<T>
   ProfScope ps(sizeof(T) == 8 ? "hop_f64_both" : "hop_f32_both",
                (double)g.V * sizeof(T) * 2 * (f->nlinks / 2 * 9 + 3 + 3));
   constexpr int S = hop_split<T>();
-#define HOP_BOTH(NL, SP)                                                                                              k_hop<T, NL, MODE, 0, false, SP, true><<<(unsigned)blocks, hop_threads(SP), 0, c.s>>>(                                  out, in, f->d, same, (T)mass, g, 0, tile, c.d_part, c.d_count, nullptr, nullptr)
+#define HOP_BOTH(NL, SP)                                                                    \
+  k_hop<T, NL, MODE, 0, false, SP, true><<<(unsigned)blocks, hop_threads(SP), 0, c.s>>>(     \
+      out, in, f->d, same, (T)mass, g, 0, tile, c.d_part, c.d_count, nullptr, nullptr)
   if (split) {
     if (f->nlinks == 16) HOP_BOTH(16, S);
     else HOP_BOTH(8, S);
@@ -539,14 +545,14 @@ void Dslash<T>::ddagd_norm2_ws(FlaT<T> *f, double mass, c2<T> *out, const c2<T> 
   // t = D_qp in (sum |t|^2 -> res[0]); out_p = m^2 in_p - D_pq t (sum |in_p|^2 -> res[1])
   if (f->nlinks == 16) {
     k_hop<T, 16, HOP_SET, 1><<<grid, HOP_BLOCK, 0, c.s>>>(tmp_block, in + par_off(g, p), f->d + q * lk_par, nullptr,
-                                                          (T)0, g, q,  0, part, count, res, nullptr);
+                                                          (T)0, g, q, 0, part, count, res, nullptr);
     k_hop<T, 16, HOP_M2_MINUS, 2><<<grid, HOP_BLOCK, 0, c.s>>>(out + par_off(g, p), tmp_block, f->d + p * lk_par,
-                                                               in + par_off(g, p), m2, g, p,  0, part, count, res + 1, nullptr);
+                                                               in + par_off(g, p), m2, g, p, 0, part, count, res + 1, nullptr);
   } else {
     k_hop<T, 8, HOP_SET, 1><<<grid, HOP_BLOCK, 0, c.s>>>(tmp_block, in + par_off(g, p), f->d + q * lk_par, nullptr,
-                                                         (T)0, g, q,  0, part, count, res, nullptr);
+                                                         (T)0, g, q, 0, part, count, res, nullptr);
     k_hop<T, 8, HOP_M2_MINUS, 2><<<grid, HOP_BLOCK, 0, c.s>>>(out + par_off(g, p), tmp_block, f->d + p * lk_par,
-                                                              in + par_off(g, p), m2, g, p,  0, part, count, res + 1, nullptr);
+                                                              in + par_off(g, p), m2, g, p, 0, part, count, res + 1, nullptr);
   }
   QLAUNCHN(2);
 }
