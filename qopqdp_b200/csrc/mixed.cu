@@ -1092,11 +1092,16 @@ k_mix_hop_q16s(uint4 *__restrict__ out, const uint4 *src, const unsigned char *_
 
 // The split hops take the place of variant 25 (the default) up to the size
 // where HBM and issue take over from latency (ms per HISQ solve, split /
-// general: 4^4 11.1 / 13.0, 4^3x8 11.8 / 13.8, 6^4 12.7 / 14.6, 8^4 13.3 / 14.8,
-// 12^4 14.7 / 16.7, 16^4 20.6 / 23.1, 16^3x20 23.6 / 24.6, 16^3x24 25.4 / 25.4,
-// 16^3x32 30.4 / 28.6).
+// general: 8^4 13.3 / 14.8, 12^4 14.7 / 16.7, 16^4 20.6 / 23.1, 16^3x20 23.6 /
+// 24.6, 16^3x24 25.4 / 25.4, 16^3x32 30.4 / 28.6).  Below 8^4 they are faster
+// too (4^4 11.1 / 13.0, 6^4 12.7 / 14.6), but their row sums round in another
+// order than those of the hop on a decomposed lattice, which has the general
+// form: on lattices that small the count of a light-mass solve scatters by
+// 4 % with the order (4x6x4x8, m 0.01, ten sources: 2653 / 2652 on average,
+// 2491-2782 / 2549-2763 singly), and a solve there keeps the count of its
+// decomposed counterpart.
 constexpr int HOP_SMALL = 32;   // the split hops in the tuner's list: no value of the option
-static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh <= 45000; }
+static bool use_q16_small(i64 Vh) { return ctx().opt.hop_kernel == 25 && Vh >= 2048 && Vh <= 45000; }
 
 template <int KIND>
 static void launch_q16_small(int nl, bool recon, float c_long, uint4 *out, const uint4 *src, const unsigned char *lk,

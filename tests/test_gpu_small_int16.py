@@ -31,7 +31,7 @@ def _links(L, kind):
 
 
 @pytest.mark.parametrize("L", [(4, 4, 4, 4), (4, 4, 4, 6), (6, 6, 6, 10), (8, 8, 8, 8), (6, 6, 10, 14),
-                               (16, 16, 16, 20), (16, 16, 18, 20)])   # the last on the general hop
+                               (16, 16, 16, 20), (16, 16, 18, 20)])   # the first three and the last: the general hop
 @pytest.mark.parametrize("kind", ["hisq", "general", "fat"])
 @pytest.mark.parametrize("eo", [0, 1])
 def test_split_hop(L, kind, eo):
