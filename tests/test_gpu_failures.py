@@ -31,9 +31,14 @@ QOP_SUCCESS, QOP_FAIL, QOP_MEM_ERROR = 0, 1, 3   # include/qop.h (reference qop_
 L8 = (8, 8, 8, 8)
 
 
+def _zero(q, fla, h):
+    for eo in (0, 1):
+        q.dslash(fla, 0.0, h, h, eo, eo)    # the mass term alone; (2, 2) would add the hop
+
+
 def _solve(q, fla, mass, hout, hin, eo, rsq=1e-20, inject=0):
     """one invert from a zero guess; inject = n makes its n-th device allocation fail"""
-    q.dslash(fla, 0.0, hout, hout, 2, 2)                    # zero guess
+    _zero(q, fla, hout)
     ia = QOP_invert_arg_t(1e9, 20000, 20000, 5, eo)
     ra = QOP_resid_arg_t(rsq, 0, 0, 0, 0, 0)
     assert q.lib.QOPB_inject_alloc_failure(inject) == 0
@@ -46,7 +51,7 @@ def _multi(q, fla, masses, hin, hout, eo, inject=0):
     ia = QOP_invert_arg_t(1e9, 20000, 20000, 5, eo)
     ras = [[QOP_resid_arg_t(1e-20, 0, 0, 0, 0, 0) for _ in masses]]
     for h in hout:
-        q.dslash(fla, 0.0, h, h, 2, 2)
+        _zero(q, fla, h)
     assert q.lib.QOPB_inject_alloc_failure(inject) == 0
     info = q.invert_multi(fla, [masses], [hout], [hin], ia, ras)
     assert q.lib.QOPB_inject_alloc_failure(0) == 0
