@@ -78,10 +78,10 @@ __global__ void __launch_bounds__(3 * ST_SITES, ST_MINB) k_naik(const __grid_con
 // 12 staples and about 25 field passes where 18 staples took about 95.  The
 // latency of the L2 reads bounds them (24^3 x 48, HISQ: the whole call 9.4 ms
 // against 22.4 with one launch per staple; 12^4: 0.44 against 1.35 ms).
-// Work fields: three S_n and three X_n.  Where six do not fit, one X_n at a
-// time is formed and added (four fields): with the finished links (eight
-// slots of FP32 are four such fields) no lattice needs more than the largest
-// sum of its outputs.
+// Work fields: three S_n and three X_n.  Where six do not fit, four: one X_n
+// at a time is formed and added.  The finished links, allocated next, are at
+// least as large (eight FP32 slots are four such fields), so the small form
+// never sets the largest lattice that a call takes.
 static double make_imp_links(const QOP_asqtad_coeffs_t *cf, const double2 *gf, const double2 *gfLong, double2 *fl,
                              double2 *ll) {
   const Geom &g = ctx().g;
